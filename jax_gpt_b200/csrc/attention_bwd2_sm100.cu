@@ -114,7 +114,7 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
   const int kv_row0 = b * a.T + jb * 128;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_desc(&tq);
       tma_prefetch_desc(&tdo);
       mbar_arrive_expect_tx(&bars->kv_full, 2 * kTile);
@@ -136,22 +136,22 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
       }
     }
   } else if (warp == 1) {
-    constexpr uint32_t idesc_st = make_idesc(128, 64, 0, 0, 1);   // K-major x K-major, 64 queries
-    constexpr uint32_t idesc_kn = make_idesc(128, D, 0, 1, 1);    // A K-major, B MN-major
-    constexpr uint32_t idesc_nn = make_idesc(128, D, 1, 1, 1);    // A MN-major, B MN-major
-    bool ok = mbar_wait(&bars->kv_full, 0, abort_flag);
-    if (!ok && lane == 0) report_status(a.status, kWaitFullTimeout, 221, jb, 0);
-    const uint32_t aK = smem_u32(smem + kOffK), aV = smem_u32(smem + kOffV);
-    const uint32_t aPT = smem_u32(smem + kOffPT);
-    // S^T and dP^T of query half `hf` (64 queries) of block `it`.
-    auto issue_scores = [&](int it, int hf) -> bool {
-      const int s = it & 1;
-      if (!mbar_wait(&bars->qdo_full[s], (it >> 1) & 1, abort_flag)) {
-        if (lane == 0) report_status(a.status, kWaitFullTimeout, 222, jb, it);
-        return false;
-      }
-      tc_fence_after();
-      if (lane == 0) {
+    if (elect_one()) {   // one thread waits and issues
+      constexpr uint32_t idesc_st = make_idesc(128, 64, 0, 0, 1);   // K-major x K-major, 64 queries
+      constexpr uint32_t idesc_kn = make_idesc(128, D, 0, 1, 1);    // A K-major, B MN-major
+      constexpr uint32_t idesc_nn = make_idesc(128, D, 1, 1, 1);    // A MN-major, B MN-major
+      bool ok = mbar_wait(&bars->kv_full, 0, abort_flag);
+      if (!ok) report_status(a.status, kWaitFullTimeout, 221, jb, 0);
+      const uint32_t aK = smem_u32(smem + kOffK), aV = smem_u32(smem + kOffV);
+      const uint32_t aPT = smem_u32(smem + kOffPT);
+      // S^T and dP^T of query half `hf` (64 queries) of block `it`.
+      auto issue_scores = [&](int it, int hf) -> bool {
+        const int s = it & 1;
+        if (!mbar_wait(&bars->qdo_full[s], (it >> 1) & 1, abort_flag)) {
+          report_status(a.status, kWaitFullTimeout, 222, jb, it);
+          return false;
+        }
+        tc_fence_after();
         const uint32_t aQ = smem_u32(smem + kOffRing + s * 2 * kTile) + hf * 8192;  // rows 64*hf.. of the tile
         const uint32_t aDO = aQ + kTile;
 #pragma unroll
@@ -163,29 +163,26 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
           umma_bf16(tmem + kColDP + hf * 64, make_smem_desc(aV + kk * 32, 16, 1024),
                     make_smem_desc(aDO + kk * 32, 16, 1024), idesc_st, kk > 0);
         tc_commit(&bars->st_full[hf]);
-      }
-      __syncwarp();
-      return true;
-    };
-    if (ok && n_iters > 0) ok = issue_scores(0, 0) && issue_scores(0, 1);
-    for (int it = 0; it < n_iters && ok; ++it) {
-      const int s = it & 1;
-      const uint32_t aQ = smem_u32(smem + kOffRing + s * 2 * kTile);
-      const uint32_t aDO = aQ + kTile;
-      const uint32_t aDST = smem_u32(smem + kOffDST + (it & 1) * 32768);
-      for (int hf = 0; hf < 2 && ok; ++hf) {
-        if (!mbar_wait(&bars->p_ready[hf], it & 1, abort_flag)) {
-          if (lane == 0) report_status(a.status, kWaitAttnTimeout, 224, jb, it);
-          ok = false;
-          break;
-        }
-        if (hf == 1 && it > 0 && !mbar_wait(&bars->dq_read, (it - 1) & 1, abort_flag)) {
-          if (lane == 0) report_status(a.status, kWaitAttnTimeout, 223, jb, it);
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-        if (lane == 0) {
+        return true;
+      };
+      if (ok && n_iters > 0) ok = issue_scores(0, 0) && issue_scores(0, 1);
+      for (int it = 0; it < n_iters && ok; ++it) {
+        const int s = it & 1;
+        const uint32_t aQ = smem_u32(smem + kOffRing + s * 2 * kTile);
+        const uint32_t aDO = aQ + kTile;
+        const uint32_t aDST = smem_u32(smem + kOffDST + (it & 1) * 32768);
+        for (int hf = 0; hf < 2 && ok; ++hf) {
+          if (!mbar_wait(&bars->p_ready[hf], it & 1, abort_flag)) {
+            report_status(a.status, kWaitAttnTimeout, 224, jb, it);
+            ok = false;
+            break;
+          }
+          if (hf == 1 && it > 0 && !mbar_wait(&bars->dq_read, (it - 1) & 1, abort_flag)) {
+            report_status(a.status, kWaitAttnTimeout, 223, jb, it);
+            ok = false;
+            break;
+          }
+          tc_fence_after();
           // contraction over the 64 queries of this half: four 16-query steps
 #pragma unroll
           for (int k4 = 0; k4 < 4; ++k4) {
@@ -207,9 +204,8 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
             tc_commit(&bars->dq_full);
             tc_commit(&bars->qdo_empty[s]);
           }
+          if (it + 1 < n_iters) ok = issue_scores(it + 1, hf);
         }
-        __syncwarp();
-        if (it + 1 < n_iters) ok = issue_scores(it + 1, hf);
       }
     }
   } else {

@@ -144,7 +144,7 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tq, const __grid_consta
   const int kv_row0 = b * a.T + jb * 128;
 
   if (warp == 0) {
-    if (lane == 0 && n_iters > 0) {
+    if (n_iters > 0 && elect_one()) {
       tma_prefetch_desc(&tq);
       tma_prefetch_desc(&tdo);
       mbar_arrive_expect_tx(&bars->kv_full, C::kKTile + C::kVTile);
@@ -183,22 +183,22 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tq, const __grid_consta
       }
     }
   } else if (warp == 1) {
-    constexpr uint32_t idesc_st = make_idesc(128, 64, 0, 0, 1);        // K-major x K-major, 64 queries
-    constexpr uint32_t idesc_dv = make_idesc(128, C::NV, 0, 1, 1);     // A K-major, B MN-major
-    constexpr uint32_t idesc_dk = make_idesc(128, C::NK, 0, 1, 1);
-    constexpr uint32_t idesc_dq = make_idesc(128, 64, 1, 1, 1);        // A MN-major (K^T), B MN-major (dS^T)
-    bool ok = n_iters > 0 && mbar_wait(&bars->kv_full, 0, abort_flag);
-    if (n_iters > 0 && !ok && lane == 0) report_status(a.status, kWaitFullTimeout, 241, jb, 0);
-    const uint32_t aK = smem_u32(smem + C::kOffK), aV = smem_u32(smem + C::kOffV);
-    const uint32_t aPT = smem_u32(smem + C::kOffPT), aDST = smem_u32(smem + C::kOffDST);
-    auto issue_scores = [&](int it) -> bool {
-      const int s = it % C::kStages;
-      if (!mbar_wait(&bars->qdo_full[s], (it / C::kStages) & 1, abort_flag)) {
-        if (lane == 0) report_status(a.status, kWaitFullTimeout, 242, jb, it);
-        return false;
-      }
-      tc_fence_after();
-      if (lane == 0) {
+    if (elect_one()) {   // one thread waits and issues
+      constexpr uint32_t idesc_st = make_idesc(128, 64, 0, 0, 1);        // K-major x K-major, 64 queries
+      constexpr uint32_t idesc_dv = make_idesc(128, C::NV, 0, 1, 1);     // A K-major, B MN-major
+      constexpr uint32_t idesc_dk = make_idesc(128, C::NK, 0, 1, 1);
+      constexpr uint32_t idesc_dq = make_idesc(128, 64, 1, 1, 1);        // A MN-major (K^T), B MN-major (dS^T)
+      bool ok = n_iters > 0 && mbar_wait(&bars->kv_full, 0, abort_flag);
+      if (n_iters > 0 && !ok) report_status(a.status, kWaitFullTimeout, 241, jb, 0);
+      const uint32_t aK = smem_u32(smem + C::kOffK), aV = smem_u32(smem + C::kOffV);
+      const uint32_t aPT = smem_u32(smem + C::kOffPT), aDST = smem_u32(smem + C::kOffDST);
+      auto issue_scores = [&](int it) -> bool {
+        const int s = it % C::kStages;
+        if (!mbar_wait(&bars->qdo_full[s], (it / C::kStages) & 1, abort_flag)) {
+          report_status(a.status, kWaitFullTimeout, 242, jb, it);
+          return false;
+        }
+        tc_fence_after();
         const uint32_t aQ = smem_u32(smem + C::kOffRing + s * C::kStageBytes);
         const uint32_t aDO = aQ + C::kQTile;
 #pragma unroll
@@ -210,23 +210,20 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tq, const __grid_consta
           umma_bf16(tmem + C::kColDP, make_smem_desc(aV + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024),
                     make_smem_desc(aDO + (kk >> 2) * 8192 + (kk & 3) * 32, 16, 1024), idesc_st, kk > 0);
         tc_commit(&bars->st_full);
-      }
-      __syncwarp();
-      return true;
-    };
-    if (ok) ok = issue_scores(0);
-    for (int it = 0; it < n_iters && ok; ++it) {
-      const int s = it % C::kStages;
-      if (!mbar_wait(&bars->p_ready, it & 1, abort_flag)) {
-        if (lane == 0) report_status(a.status, kWaitAttnTimeout, 244, jb, it);
-        break;
-      }
-      if (!C::kAliasDq && it > 0 && !mbar_wait(&bars->dq_read, (it - 1) & 1, abort_flag)) {
-        if (lane == 0) report_status(a.status, kWaitAttnTimeout, 243, jb, it);
-        break;
-      }
-      tc_fence_after();
-      if (lane == 0) {
+        return true;
+      };
+      if (ok) ok = issue_scores(0);
+      for (int it = 0; it < n_iters && ok; ++it) {
+        const int s = it % C::kStages;
+        if (!mbar_wait(&bars->p_ready, it & 1, abort_flag)) {
+          report_status(a.status, kWaitAttnTimeout, 244, jb, it);
+          break;
+        }
+        if (!C::kAliasDq && it > 0 && !mbar_wait(&bars->dq_read, (it - 1) & 1, abort_flag)) {
+          report_status(a.status, kWaitAttnTimeout, 243, jb, it);
+          break;
+        }
+        tc_fence_after();
         const uint32_t aQ = smem_u32(smem + C::kOffRing + s * C::kStageBytes);
         const uint32_t aDO = aQ + C::kQTile;
         // contraction over the 64 queries of the tile: four 16-query steps
@@ -249,14 +246,13 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tq, const __grid_consta
         }
         tc_commit(&bars->dq_full);
         tc_commit(&bars->qdo_empty[s]);
-      }
-      __syncwarp();
-      if (it + 1 < n_iters) {
-        if (C::kAliasDq && !mbar_wait(&bars->dq_read, it & 1, abort_flag)) {
-          if (lane == 0) report_status(a.status, kWaitAttnTimeout, 245, jb, it);
-          break;
+        if (it + 1 < n_iters) {
+          if (C::kAliasDq && !mbar_wait(&bars->dq_read, it & 1, abort_flag)) {
+            report_status(a.status, kWaitAttnTimeout, 245, jb, it);
+            break;
+          }
+          ok = issue_scores(it + 1);
         }
-        ok = issue_scores(it + 1);
       }
     }
   } else {

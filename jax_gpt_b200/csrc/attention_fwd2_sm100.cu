@@ -125,7 +125,6 @@ struct MmaCtx {
   volatile int* abort_flag;
   int* status;
   uint32_t tmem;
-  int lane;
   uint64_t dK0, dV0, dP[2];   // descriptors of ring stage 0 / of the two P tiles
 };
 
@@ -138,21 +137,18 @@ __device__ __forceinline__ bool mma_issue_s(const MmaCtx<D>& c, uint64_t dQ, uin
   using C = Fwd2Cfg<D>;
   if (!mbar_wait(&c.bars->k_full[st], ph, c.abort_flag) ||
       (ns > 0 && !mbar_wait(&c.bars->s_free[G], (ns - 1) & 1, c.abort_flag))) {
-    if (c.lane == 0) report_status(c.status, kWaitFullTimeout, 113, G, static_cast<int>(ns));
+    report_status(c.status, kWaitFullTimeout, 113, G, static_cast<int>(ns));
     return false;
   }
   tc_fence_after();
-  if (c.lane == 0) {
-    constexpr uint32_t idesc_s = make_idesc(128, 128, 0, 0, 1);
-    const uint64_t dK = c.dK0 + static_cast<uint64_t>(st) * (C::kTile >> 4);
+  constexpr uint32_t idesc_s = make_idesc(128, 128, 0, 0, 1);
+  const uint64_t dK = c.dK0 + static_cast<uint64_t>(st) * (C::kTile >> 4);
 #pragma unroll
-    for (int kk = 0; kk < D / 16; ++kk)
-      umma_bf16(c.tmem + C::kColS + G * 128, dQ + 2 * kk, dK + 2 * kk, idesc_s, kk > 0);
-    tc_commit(&c.bars->s_full[G]);
-    tc_commit(&c.bars->k_empty[st]);
-    if (q_empty != nullptr) tc_commit(q_empty);
-  }
-  __syncwarp();
+  for (int kk = 0; kk < D / 16; ++kk)
+    umma_bf16(c.tmem + C::kColS + G * 128, dQ + 2 * kk, dK + 2 * kk, idesc_s, kk > 0);
+  tc_commit(&c.bars->s_full[G]);
+  tc_commit(&c.bars->k_empty[st]);
+  if (q_empty != nullptr) tc_commit(q_empty);
   ++ns;
   return true;
 }
@@ -165,22 +161,19 @@ __device__ __forceinline__ bool mma_issue_pv(const MmaCtx<D>& c, uint32_t st, ui
   using C = Fwd2Cfg<D>;
   if (!mbar_wait(&c.bars->v_full[st], ph, c.abort_flag) || !mbar_wait(&c.bars->p_ready[G], npv & 1, c.abort_flag) ||
       (wait_o_free && !mbar_wait(&c.bars->o_free[G], (n_items_done - 1) & 1, c.abort_flag))) {
-    if (c.lane == 0) report_status(c.status, kWaitAttnTimeout, 114, G, static_cast<int>(npv));
+    report_status(c.status, kWaitAttnTimeout, 114, G, static_cast<int>(npv));
     return false;
   }
   tc_fence_after();
-  if (c.lane == 0) {
-    constexpr uint32_t idesc_o = make_idesc(128, D, 0, 1, 1);
-    const uint64_t dV = c.dV0 + static_cast<uint64_t>(st) * (C::kTile >> 4);
-    const uint64_t dP = c.dP[G];
+  constexpr uint32_t idesc_o = make_idesc(128, D, 0, 1, 1);
+  const uint64_t dV = c.dV0 + static_cast<uint64_t>(st) * (C::kTile >> 4);
+  const uint64_t dP = c.dP[G];
 #pragma unroll
-    for (int kk = 0; kk < 8; ++kk)
-      umma_bf16(c.tmem + C::kColO + G * D, dP + ((kk >> 2) * 1024 + (kk & 3) * 2), dV + kk * 128, idesc_o,
-                accumulate || kk > 0);
-    tc_commit(&c.bars->o_full[G]);
-    tc_commit(&c.bars->v_empty[st]);
-  }
-  __syncwarp();
+  for (int kk = 0; kk < 8; ++kk)
+    umma_bf16(c.tmem + C::kColO + G * D, dP + ((kk >> 2) * 1024 + (kk & 3) * 2), dV + kk * 128, idesc_o,
+              accumulate || kk > 0);
+  tc_commit(&c.bars->o_full[G]);
+  tc_commit(&c.bars->v_empty[st]);
   ++npv;
   return true;
 }
@@ -190,8 +183,7 @@ __device__ __forceinline__ bool mma_issue_pv(const MmaCtx<D>& c, uint32_t st, ui
 template <int D>
 __device__ __forceinline__ bool mma_skip_stage(const MmaCtx<D>& c, uint64_t* full, uint64_t* empty, uint32_t ph) {
   if (!mbar_wait(full, ph, c.abort_flag)) return false;
-  if (c.lane == 0) mbar_arrive(empty);
-  __syncwarp();
+  mbar_arrive(empty);
   return true;
 }
 
@@ -209,7 +201,7 @@ __device__ __forceinline__ void mma_loop(MmaCtx<D>& c, const Fwd2Args& a, uint32
     const int n_g = it.nkv[G], n_max = it.n_max;
     const int slot = li & 1;
     if (!mbar_wait(&bars->q_full[slot], (li >> 1) & 1, c.abort_flag)) {
-      if (c.lane == 0) report_status(c.status, kWaitFullTimeout, 112, idx, G);
+      report_status(c.status, kWaitFullTimeout, 112, idx, G);
       break;
     }
     const uint64_t dQ = make_smem_desc(sb + C::kOffQ + (slot * 2 + G) * C::kTile, 16, 1024);
@@ -217,8 +209,7 @@ __device__ __forceinline__ void mma_loop(MmaCtx<D>& c, const Fwd2Args& a, uint32
     if (n_g > 0) {
       ok = mma_issue_s<D, G>(c, dQ, st, ph, ns, n_g == 1 ? q_empty : nullptr);
     } else {
-      if (c.lane == 0) mbar_arrive(q_empty);
-      __syncwarp();
+      mbar_arrive(q_empty);
       ok = mma_skip_stage<D>(c, &bars->k_full[st], &bars->k_empty[st], ph);
     }
     for (int j = 0; j < n_max && ok; ++j) {
@@ -289,7 +280,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
   // One instruction for the whole third warpgroup (setmaxnreg is warpgroup-aligned): it gives registers up ...
   asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
   if (warp == kWarpTma) {
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_desc(&tq);
       tma_prefetch_desc(&tk);
       tma_prefetch_desc(&tv);
@@ -338,14 +329,15 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
     c.abort_flag = abort_flag;
     c.status = a.status;
     c.tmem = tmem;
-    c.lane = lane;
     const uint32_t sb = smem_u32(smem);
     c.dK0 = make_smem_desc(sb + C::kOffK, 16, 1024);
     c.dV0 = make_smem_desc(sb + C::kOffV, 16384, 1024);
     c.dP[0] = make_smem_desc(sb + C::kOffP, 16, 1024);
     c.dP[1] = make_smem_desc(sb + C::kOffP + C::kPBytes, 16, 1024);
-    if (warp == kWarpMma) mma_loop<D, 0>(c, a, sb);
-    else mma_loop<D, 1>(c, a, sb);
+    if (elect_one()) {   // one thread waits and issues
+      if (warp == kWarpMma) mma_loop<D, 0>(c, a, sb);
+      else mma_loop<D, 1>(c, a, sb);
+    }
   }
   } else {
     // ... and the two softmax warpgroups take them.

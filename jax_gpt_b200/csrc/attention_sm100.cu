@@ -153,7 +153,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
   uint8_t* sP = smem + C::kOffP;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_arrive_expect_tx(&bars->q_full, C::kQTile);
       load_tile<D>(sQ, &tq, &bars->q_full, h * D, row0);
       for (int j = 0; j < n_kv; ++j) {
@@ -171,36 +171,33 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
       }
     }
   } else if (warp == 1) {
-    constexpr uint32_t idesc_s = make_idesc(128, 128, 0, 0, 1);
-    constexpr uint32_t idesc_o = make_idesc(128, DV, 0, 1, 1);
-    bool ok = mbar_wait(&bars->q_full, 0, abort_flag);
-    if (!ok && lane == 0) report_status(a.status, kWaitFullTimeout, 101, blockIdx.z, 0);
-    for (int j = 0; j < n_kv && ok; ++j) {
-      const int s = j % C::kStages;
-      const uint32_t ph = (j / C::kStages) & 1;
-      if (!mbar_wait(&bars->kv_full[s], ph, abort_flag)) {
-        if (lane == 0) report_status(a.status, kWaitFullTimeout, 102, blockIdx.z, j);
-        break;
-      }
-      tc_fence_after();
-      const uint32_t aQ = smem_u32(sQ);
-      const uint32_t aK = smem_u32(smem + C::kOffK + s * C::kStageBytes);
-      const uint32_t aV = aK + C::kQTile;
-      if (lane == 0) {
+    if (elect_one()) {   // one thread waits and issues
+      constexpr uint32_t idesc_s = make_idesc(128, 128, 0, 0, 1);
+      constexpr uint32_t idesc_o = make_idesc(128, DV, 0, 1, 1);
+      bool ok = mbar_wait(&bars->q_full, 0, abort_flag);
+      if (!ok) report_status(a.status, kWaitFullTimeout, 101, blockIdx.z, 0);
+      for (int j = 0; j < n_kv && ok; ++j) {
+        const int s = j % C::kStages;
+        const uint32_t ph = (j / C::kStages) & 1;
+        if (!mbar_wait(&bars->kv_full[s], ph, abort_flag)) {
+          report_status(a.status, kWaitFullTimeout, 102, blockIdx.z, j);
+          break;
+        }
+        tc_fence_after();
+        const uint32_t aQ = smem_u32(sQ);
+        const uint32_t aK = smem_u32(smem + C::kOffK + s * C::kStageBytes);
+        const uint32_t aV = aK + C::kQTile;
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk) {
           const uint32_t off = (kk >> 2) * 16384 + (kk & 3) * 32;
           umma_bf16(tmem, make_smem_desc(aQ + off, 16, 1024), make_smem_desc(aK + off, 16, 1024), idesc_s, kk > 0);
         }
         tc_commit(&bars->s_full);
-      }
-      __syncwarp();
-      if (!mbar_wait(&bars->p_ready, j & 1, abort_flag)) {
-        if (lane == 0) report_status(a.status, kWaitAttnTimeout, 103, blockIdx.z, j);
-        break;
-      }
-      tc_fence_after();
-      if (lane == 0) {
+        if (!mbar_wait(&bars->p_ready, j & 1, abort_flag)) {
+          report_status(a.status, kWaitAttnTimeout, 103, blockIdx.z, j);
+          break;
+        }
+        tc_fence_after();
         const uint32_t aP = smem_u32(sP);
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk) {
@@ -211,7 +208,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
         tc_commit(&bars->o_full);
         tc_commit(&bars->kv_empty[s]);
       }
-      __syncwarp();
     }
   } else {
     // Eight softmax warps: warps w and w+4 share a TMEM lane quarter (the same 32 query rows)
@@ -446,7 +442,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
   const int kv_row0 = b * a.T + jb * 128;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_arrive_expect_tx(&bars->kv_full, 2 * C::kTile);
       load_tile<D>(smem + C::kOffK, &tk, &bars->kv_full, hkv * D, kv_row0);
       load_tile<D>(smem + C::kOffV, &tv, &bars->kv_full, hkv * D, kv_row0);
@@ -466,25 +462,25 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
       }
     }
   } else if (warp == 1) {
-    constexpr uint32_t idesc_st = make_idesc(128, 128, 0, 0, 1);  // K-major x K-major
-    constexpr uint32_t idesc_kn = make_idesc(128, D, 0, 1, 1);    // A K-major, B MN-major
-    constexpr uint32_t idesc_nn = make_idesc(128, D, 1, 1, 1);    // A MN-major, B MN-major
-    bool ok = mbar_wait(&bars->kv_full, 0, abort_flag);
-    if (!ok && lane == 0) report_status(a.status, kWaitFullTimeout, 201, blockIdx.z, 0);
-    const uint32_t aK = smem_u32(smem + C::kOffK), aV = smem_u32(smem + C::kOffV);
-    const uint32_t aPT = smem_u32(smem + C::kOffPT), aDST = smem_u32(smem + C::kOffDST);
-    // S^T = K Q^T and dP^T = V dO^T of iteration `it` (its Q / dO stage must have landed).
-    auto issue_scores = [&](int it) -> bool {
-      const int s = it % C::kStages;
-      const uint32_t ph = (it / C::kStages) & 1;
-      if (!mbar_wait(&bars->qdo_full[s], ph, abort_flag)) {
-        if (lane == 0) report_status(a.status, kWaitFullTimeout, 202, blockIdx.z, it);
-        return false;
-      }
-      tc_fence_after();
-      const uint32_t aQ = smem_u32(smem + C::kOffRing + s * 2 * C::kTile);
-      const uint32_t aDO = aQ + C::kTile;
-      if (lane == 0) {
+    if (elect_one()) {   // one thread waits and issues
+      constexpr uint32_t idesc_st = make_idesc(128, 128, 0, 0, 1);  // K-major x K-major
+      constexpr uint32_t idesc_kn = make_idesc(128, D, 0, 1, 1);    // A K-major, B MN-major
+      constexpr uint32_t idesc_nn = make_idesc(128, D, 1, 1, 1);    // A MN-major, B MN-major
+      bool ok = mbar_wait(&bars->kv_full, 0, abort_flag);
+      if (!ok) report_status(a.status, kWaitFullTimeout, 201, blockIdx.z, 0);
+      const uint32_t aK = smem_u32(smem + C::kOffK), aV = smem_u32(smem + C::kOffV);
+      const uint32_t aPT = smem_u32(smem + C::kOffPT), aDST = smem_u32(smem + C::kOffDST);
+      // S^T = K Q^T and dP^T = V dO^T of iteration `it` (its Q / dO stage must have landed).
+      auto issue_scores = [&](int it) -> bool {
+        const int s = it % C::kStages;
+        const uint32_t ph = (it / C::kStages) & 1;
+        if (!mbar_wait(&bars->qdo_full[s], ph, abort_flag)) {
+          report_status(a.status, kWaitFullTimeout, 202, blockIdx.z, it);
+          return false;
+        }
+        tc_fence_after();
+        const uint32_t aQ = smem_u32(smem + C::kOffRing + s * 2 * C::kTile);
+        const uint32_t aDO = aQ + C::kTile;
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk) {
           const uint32_t off = (kk >> 2) * 16384 + (kk & 3) * 32;
@@ -497,21 +493,18 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
                     kk > 0);
         }
         tc_commit(&bars->st_full);
-      }
-      __syncwarp();
-      return true;
-    };
-    if (ok && n_iters > 0) ok = issue_scores(0);
-    for (int it = 0; it < n_iters && ok; ++it) {
-      const int s = it % C::kStages;
-      if (!mbar_wait(&bars->p_ready, it & 1, abort_flag)) {
-        if (lane == 0) report_status(a.status, kWaitAttnTimeout, 204, blockIdx.z, it);
-        break;
-      }
-      tc_fence_after();
-      const uint32_t aQ = smem_u32(smem + C::kOffRing + s * 2 * C::kTile);
-      const uint32_t aDO = aQ + C::kTile;
-      if (lane == 0) {
+        return true;
+      };
+      if (ok && n_iters > 0) ok = issue_scores(0);
+      for (int it = 0; it < n_iters && ok; ++it) {
+        const int s = it % C::kStages;
+        if (!mbar_wait(&bars->p_ready, it & 1, abort_flag)) {
+          report_status(a.status, kWaitAttnTimeout, 204, blockIdx.z, it);
+          break;
+        }
+        tc_fence_after();
+        const uint32_t aQ = smem_u32(smem + C::kOffRing + s * 2 * C::kTile);
+        const uint32_t aDO = aQ + C::kTile;
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk) {  // contraction over the 128 query rows
           const uint32_t off = (kk >> 2) * 16384 + (kk & 3) * 32;
@@ -531,16 +524,15 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
         }
         tc_commit(&bars->dq_full);
         tc_commit(&bars->qdo_empty[s]);
-      }
-      __syncwarp();
-      if (it + 1 < n_iters) {
-        if (kAliasDq && !mbar_wait(&bars->dq_read, it & 1, abort_flag)) {
-          if (lane == 0) report_status(a.status, kWaitAttnTimeout, 203, blockIdx.z, it);
-          break;
+        if (it + 1 < n_iters) {
+          if (kAliasDq && !mbar_wait(&bars->dq_read, it & 1, abort_flag)) {
+            report_status(a.status, kWaitAttnTimeout, 203, blockIdx.z, it);
+            break;
+          }
+          // P^T / dS^T of `it` are only re-written after the compute warps have seen dq_full(it),
+          // i.e. after the MMAs above have finished reading them.
+          ok = issue_scores(it + 1);
         }
-        // P^T / dS^T of `it` are only re-written after the compute warps have seen dq_full(it),
-        // i.e. after the MMAs above have finished reading them.
-        ok = issue_scores(it + 1);
       }
     }
   } else {

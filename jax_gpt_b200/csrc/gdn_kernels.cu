@@ -101,7 +101,7 @@ gdn_scan_kernel(const __grid_constant__ CUtensorMap t_kq, const __grid_constant_
   const uint32_t tmem = bars->tmem_base;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       bool ok = true;
       int issued = 0;
       for (int n = 0; n < N; ++n, ++issued) {
@@ -132,31 +132,28 @@ gdn_scan_kernel(const __grid_constant__ CUtensorMap t_kq, const __grid_constant_
       }
     }
   } else if (warp == 1) {
-    constexpr uint32_t idesc_kn = make_idesc(128, 128, 0, 1, 1);   // A K-major, B MN-major
-    constexpr uint32_t idesc_nn = make_idesc(128, 128, 1, 1, 1);   // both MN-major
-    const uint32_t a_sb = smem_u32(sb), a_vn = smem_u32(vn);
-    for (int n = 0; n < N; ++n) {
-      const int st = n & 1;
-      const uint32_t a1 = smem_u32(smem + st * kStageBytes), a2 = a1 + kA1Bytes, kd = a2 + kA2Bytes;
-      if (!mbar_wait(&bars->s_ready, n & 1, abort_flag) || !mbar_wait(&bars->full[st], (n >> 1) & 1, abort_flag)) {
-        if (lane == 0) report_status(a.status, kWaitFullTimeout, 101, bh, n);
-        break;
-      }
-      tc_fence_after();
-      if (lane == 0) {
+    if (elect_one()) {   // one thread waits and issues
+      constexpr uint32_t idesc_kn = make_idesc(128, 128, 0, 1, 1);   // A K-major, B MN-major
+      constexpr uint32_t idesc_nn = make_idesc(128, 128, 1, 1, 1);   // both MN-major
+      const uint32_t a_sb = smem_u32(sb), a_vn = smem_u32(vn);
+      for (int n = 0; n < N; ++n) {
+        const int st = n & 1;
+        const uint32_t a1 = smem_u32(smem + st * kStageBytes), a2 = a1 + kA1Bytes, kd = a2 + kA2Bytes;
+        if (!mbar_wait(&bars->s_ready, n & 1, abort_flag) || !mbar_wait(&bars->full[st], (n >> 1) & 1, abort_flag)) {
+          report_status(a.status, kWaitFullTimeout, 101, bh, n);
+          break;
+        }
+        tc_fence_after();
 #pragma unroll
         for (int k = 0; k < 8; ++k)   // K = dk = 128: block k / 4, 32 bytes per step
           umma_bf16(tmem, make_smem_desc(a1 + (k >> 2) * 16384 + (k & 3) * 32, 16, 1024),
                     make_smem_desc(a_sb + k * 2048, 16384, 1024), idesc_kn, k > 0 ? 1u : 0u);
         tc_commit(&bars->d_full);
-      }
-      __syncwarp();
-      if (!mbar_wait(&bars->vn_ready, n & 1, abort_flag)) {
-        if (lane == 0) report_status(a.status, kWaitFullTimeout, 102, bh, n);
-        break;
-      }
-      tc_fence_after();
-      if (lane == 0) {
+        if (!mbar_wait(&bars->vn_ready, n & 1, abort_flag)) {
+          report_status(a.status, kWaitFullTimeout, 102, bh, n);
+          break;
+        }
+        tc_fence_after();
 #pragma unroll
         for (int k = 0; k < 4; ++k)   // K = 64 tokens
           umma_bf16(tmem, make_smem_desc(a2 + k * 32, 16, 1024), make_smem_desc(a_vn + k * 2048, 8192, 1024), idesc_kn, 1u);
@@ -167,7 +164,6 @@ gdn_scan_kernel(const __grid_constant__ CUtensorMap t_kq, const __grid_constant_
         tc_commit(&bars->empty[st]);
         tc_commit(&bars->p_full);
       }
-      __syncwarp();
     }
   } else {
     const int q = warp & 3;
@@ -678,7 +674,7 @@ gdn_scan_bwd_kernel(const __grid_constant__ BwdMaps tm, const __grid_constant__ 
   constexpr uint32_t kT1 = 0, kT2 = 128, kT3 = 256, kT4 = 320;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       int it = 0;
       for (int n = N - 1; n >= 0; --n, ++it) {
         // the previous chunk's products are done with the tiles (inputs_free) AND its epilogue has finished
@@ -709,21 +705,21 @@ gdn_scan_bwd_kernel(const __grid_constant__ BwdMaps tm, const __grid_constant__ 
       }
     }
   } else if (warp == 1) {
-    constexpr uint32_t i_kn = make_idesc(128, 128, 0, 1, 1);   // A K-major, B MN-major
-    constexpr uint32_t i_nn = make_idesc(128, 128, 1, 1, 1);   // both MN-major
-    constexpr uint32_t i_kk = make_idesc(128, 128, 0, 0, 1);   // both K-major
-    constexpr uint32_t i_kk64 = make_idesc(128, 64, 0, 0, 1);
-    const uint32_t b0 = smem_u32(smem);
-    const uint32_t kq = b0 + kTileKq, kd = b0 + kTileKd, in = b0 + kTileIn, dw = b0 + kTileDw, ss = b0 + kTileS,
-                   vn = b0 + kTileVn, ds = b0 + kTileDs;
-    int it = 0;
-    for (int n = N - 1; n >= 0; --n, ++it) {
-      if (!mbar_wait(&bars->ds_ready, it & 1, abort_flag) || !mbar_wait(&bars->full, it & 1, abort_flag)) {
-        if (lane == 0) report_status(a.status, kWaitFullTimeout, 121, bh, n);
-        break;
-      }
-      tc_fence_after();
-      if (lane == 0) {
+    if (elect_one()) {   // one thread waits and issues
+      constexpr uint32_t i_kn = make_idesc(128, 128, 0, 1, 1);   // A K-major, B MN-major
+      constexpr uint32_t i_nn = make_idesc(128, 128, 1, 1, 1);   // both MN-major
+      constexpr uint32_t i_kk = make_idesc(128, 128, 0, 0, 1);   // both K-major
+      constexpr uint32_t i_kk64 = make_idesc(128, 64, 0, 0, 1);
+      const uint32_t b0 = smem_u32(smem);
+      const uint32_t kq = b0 + kTileKq, kd = b0 + kTileKd, in = b0 + kTileIn, dw = b0 + kTileDw, ss = b0 + kTileS,
+                     vn = b0 + kTileVn, ds = b0 + kTileDs;
+      int it = 0;
+      for (int n = N - 1; n >= 0; --n, ++it) {
+        if (!mbar_wait(&bars->ds_ready, it & 1, abort_flag) || !mbar_wait(&bars->full, it & 1, abort_flag)) {
+          report_status(a.status, kWaitFullTimeout, 121, bh, n);
+          break;
+        }
+        tc_fence_after();
 #pragma unroll
         for (int k = 0; k < 8; ++k)   // T1 = [kdec ; 0] dS      (K = dk)
           umma_bf16(tmem + kT1, make_smem_desc(kd + (k >> 2) * 16384 + (k & 3) * 32, 16, 1024),
@@ -733,14 +729,11 @@ gdn_scan_bwd_kernel(const __grid_constant__ BwdMaps tm, const __grid_constant__ 
           umma_bf16(tmem + kT1, make_smem_desc(in + k * 2048, 8192, 1024), make_smem_desc(dw + k * 2048, 16384, 1024),
                     i_nn, 1u);
         tc_commit(&bars->t1_full);
-      }
-      __syncwarp();
-      if (!mbar_wait(&bars->w_ready, it & 1, abort_flag)) {
-        if (lane == 0) report_status(a.status, kWaitFullTimeout, 122, bh, n);
-        break;
-      }
-      tc_fence_after();
-      if (lane == 0) {
+        if (!mbar_wait(&bars->w_ready, it & 1, abort_flag)) {
+          report_status(a.status, kWaitFullTimeout, 122, bh, n);
+          break;
+        }
+        tc_fence_after();
 #pragma unroll
         for (int k = 0; k < 8; ++k) {   // K = dv
           const uint64_t a_dw = make_smem_desc(dw + (k >> 2) * 16384 + (k & 3) * 32, 16, 1024);
@@ -760,7 +753,6 @@ gdn_scan_bwd_kernel(const __grid_constant__ BwdMaps tm, const __grid_constant__ 
         tc_commit(&bars->inputs_free);
         tc_commit(&bars->t2_full);
       }
-      __syncwarp();
     }
   } else {
     const int q = warp & 3;

@@ -76,7 +76,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ 
   const uint32_t tmem_base = bars->tmem_base;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -109,22 +109,22 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ 
       }
     }
   } else if (warp == 1) {
-    constexpr uint32_t idesc = make_idesc(BM, BN, 0, 0, /*e4m3*/ 0);
-    int stage = 0;
-    uint32_t phase = 0;
-    int slab_iter = 0;  // global slab counter: buffer = slab_iter & 1
-    bool ok = true;
-    for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
-      for (int s = 0; s < slabs && ok; ++s, ++slab_iter) {
-        const int buf = slab_iter & 1;
-        if (!mbar_wait(&bars->tmem_empty[buf], ((slab_iter >> 1) & 1) ^ 1, abort_flag) ||
-            !mbar_wait(&bars->full[stage], phase, abort_flag)) {
-          if (lane == 0) report_status(a.status, kWaitFullTimeout, 61, blockIdx.x, t);
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-        if (lane == 0) {
+    if (elect_one()) {   // one thread waits and issues
+      constexpr uint32_t idesc = make_idesc(BM, BN, 0, 0, /*e4m3*/ 0);
+      int stage = 0;
+      uint32_t phase = 0;
+      int slab_iter = 0;  // global slab counter: buffer = slab_iter & 1
+      bool ok = true;
+      for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
+        for (int s = 0; s < slabs && ok; ++s, ++slab_iter) {
+          const int buf = slab_iter & 1;
+          if (!mbar_wait(&bars->tmem_empty[buf], ((slab_iter >> 1) & 1) ^ 1, abort_flag) ||
+              !mbar_wait(&bars->full[stage], phase, abort_flag)) {
+            report_status(a.status, kWaitFullTimeout, 61, blockIdx.x, t);
+            ok = false;
+            break;
+          }
+          tc_fence_after();
           const uint32_t sa = smem_u32(smem + stage * kStageBytes), sb = sa + kTile;
 #pragma unroll
           for (int k = 0; k < BK / 32; ++k)
@@ -132,11 +132,10 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ 
                     idesc, k > 0 ? 1u : 0u);
           tc_commit(&bars->empty[stage]);
           tc_commit(&bars->tmem_full[buf]);
-        }
-        __syncwarp();
-        if (++stage == kStages) {
-          stage = 0;
-          phase ^= 1;
+          if (++stage == kStages) {
+            stage = 0;
+            phase ^= 1;
+          }
         }
       }
     }

@@ -95,7 +95,7 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant_
   const uint32_t tmem_base = bars->tmem_base;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -136,23 +136,23 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant_
       }
     }
   } else if (warp == 1) {
-    int stage = 0, iter = 0;
-    uint32_t phase = 0;
-    bool ok = true;
-    for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++iter) {
-      if (!mbar_wait(&bars->tmem_empty, (iter & 1) ^ 1, abort_flag)) {
-        if (lane == 0) report_status(a.status, kWaitTmemEmptyTimeout, 81, blockIdx.x, t);
-        break;
-      }
-      tc_fence_after();
-      for (int s = 0; s < slabs; ++s) {
-        if (!mbar_wait(&bars->full[stage], phase, abort_flag)) {
-          if (lane == 0) report_status(a.status, kWaitFullTimeout, 82, blockIdx.x, t);
-          ok = false;
+    if (elect_one()) {   // one thread waits and issues
+      int stage = 0, iter = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++iter) {
+        if (!mbar_wait(&bars->tmem_empty, (iter & 1) ^ 1, abort_flag)) {
+          report_status(a.status, kWaitTmemEmptyTimeout, 81, blockIdx.x, t);
           break;
         }
         tc_fence_after();
-        if (lane == 0) {
+        for (int s = 0; s < slabs; ++s) {
+          if (!mbar_wait(&bars->full[stage], phase, abort_flag)) {
+            report_status(a.status, kWaitFullTimeout, 82, blockIdx.x, t);
+            ok = false;
+            break;
+          }
+          tc_fence_after();
           const uint32_t sa = smem_u32(smem + stage * kStageBytes), sb = sa + kABytes;
           const uint32_t sf = smem_u32(sf_smem + stage * kStageSf);
           const uint32_t tsf = tmem_base + kSfCol0 + stage * 12;
@@ -164,15 +164,13 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant_
             umma_mxf8(tmem_base, make_smem_desc(sa + k * 32, 16, 1024), make_smem_desc(sb + k * 32, 16, 1024),
                       make_idesc_mx(BM, BN, k), tsf, tsf + 4, (s > 0 || k > 0) ? 1u : 0u);
           tc_commit(&bars->empty[stage]);
+          if (++stage == kStages) {
+            stage = 0;
+            phase ^= 1;
+          }
         }
-        __syncwarp();
-        if (++stage == kStages) {
-          stage = 0;
-          phase ^= 1;
-        }
+        if (ok) tc_commit(&bars->tmem_full);
       }
-      if (ok && lane == 0) tc_commit(&bars->tmem_full);
-      __syncwarp();
     }
   } else {
     const int ew = warp - 2;            // 0..7

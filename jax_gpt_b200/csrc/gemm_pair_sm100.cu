@@ -173,7 +173,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
 
   if (warp == 0) {
     // ------------------------------ TMA producer (both CTAs) ------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_desc(&tma_a);
       tma_prefetch_desc(&tma_b);
       const uint32_t full_leader = mapa_u32(smem_u32(&bars->full[0]), 0);
@@ -229,35 +229,35 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
       }
     }
   } else if (warp == 1) {
-    // ------------------------------ MMA issuer (leader CTA) ------------------------------
-    if (rank == 0) {
-      constexpr uint32_t idesc = make_idesc(2 * BM, BN, A_MAJOR, B_MAJOR, /*bf16*/ 1);
-      int stage = 0;
-      uint32_t phase = 0;
-      int iter = 0;
-      bool ok = true;
-      for (int t = pair; t < num_tiles && ok; t += n_pairs, ++iter) {
-        int m_blk, n_blk, ks;
-        decode_tile(t, m_blk, n_blk, ks);
-        const int acc = iter & 1;
-        const uint32_t acc_phase = (iter >> 1) & 1;
-        if (!mbar_wait(&bars->tmem_empty[acc], acc_phase ^ 1, abort_flag)) {
-          if (lane == 0) report_status(args.status, kWaitTmemEmptyTimeout, blockIdx.x, t, iter);
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-        const uint32_t tmem_d = tmem_base + acc * BN;
-        const int kb0 = ks * kb_per_split;
-        const int kb1 = min(total_kb, kb0 + kb_per_split);
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(&bars->full[stage], phase, abort_flag)) {
-            if (lane == 0) report_status(args.status, kWaitFullTimeout, blockIdx.x, t, kb);
+    if (elect_one()) {   // one thread waits and issues
+      // ------------------------------ MMA issuer (leader CTA) ------------------------------
+      if (rank == 0) {
+        constexpr uint32_t idesc = make_idesc(2 * BM, BN, A_MAJOR, B_MAJOR, /*bf16*/ 1);
+        int stage = 0;
+        uint32_t phase = 0;
+        int iter = 0;
+        bool ok = true;
+        for (int t = pair; t < num_tiles && ok; t += n_pairs, ++iter) {
+          int m_blk, n_blk, ks;
+          decode_tile(t, m_blk, n_blk, ks);
+          const int acc = iter & 1;
+          const uint32_t acc_phase = (iter >> 1) & 1;
+          if (!mbar_wait(&bars->tmem_empty[acc], acc_phase ^ 1, abort_flag)) {
+            report_status(args.status, kWaitTmemEmptyTimeout, blockIdx.x, t, iter);
             ok = false;
             break;
           }
           tc_fence_after();
-          if (lane == 0) {
+          const uint32_t tmem_d = tmem_base + acc * BN;
+          const int kb0 = ks * kb_per_split;
+          const int kb1 = min(total_kb, kb0 + kb_per_split);
+          for (int kb = kb0; kb < kb1; ++kb) {
+            if (!mbar_wait(&bars->full[stage], phase, abort_flag)) {
+              report_status(args.status, kWaitFullTimeout, blockIdx.x, t, kb);
+              ok = false;
+              break;
+            }
+            tc_fence_after();
             const uint32_t sa = smem_u32(smem + stage * kStageBytes);
             const uint32_t sb = sa + kABytes;
 #pragma unroll
@@ -269,15 +269,13 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
               umma_bf16_pair(tmem_d, adesc, bdesc, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
             }
             tc_commit_pair(&bars->empty[stage]);  // frees the stage in both CTAs
+            if (++stage == kStages) {
+              stage = 0;
+              phase ^= 1;
+            }
           }
-          __syncwarp();
-          if (++stage == kStages) {
-            stage = 0;
-            phase ^= 1;
-          }
+          if (ok) tc_commit_pair(&bars->tmem_full[acc]);
         }
-        if (ok && lane == 0) tc_commit_pair(&bars->tmem_full[acc]);
-        __syncwarp();
       }
     }
   } else {

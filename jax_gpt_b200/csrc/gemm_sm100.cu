@@ -279,7 +279,7 @@ gemm_bf16_kernel(const __grid_constant__ TmaSet tma_a, const __grid_constant__ T
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_desc(&tma_b.m[0]);
       int stage = 0;
       uint32_t phase = 0;
@@ -370,54 +370,51 @@ gemm_bf16_kernel(const __grid_constant__ TmaSet tma_a, const __grid_constant__ T
       }
     }
   } else if (warp == 1) {
-    // ------------------------------ MMA issuer ------------------------------
-    constexpr uint32_t idesc = make_idesc(BM, BN, A_MAJOR, B_MAJOR, /*bf16*/ 1);
-    int stage = 0;
-    uint32_t phase = 0;
-    int iter = 0;
-    bool ok = true;
-    for (int t = blockIdx.x; t < num_tiles && ok; t += gemm_ctas, ++iter) {
-      int m_blk, n_blk, ks;
-      decode_tile(t, m_blk, n_blk, ks);
-      const int acc = iter & 1;
-      const uint32_t acc_phase = (iter >> 1) & 1;
-      if (!mbar_wait(&bars->tmem_empty[acc], acc_phase ^ 1, abort_flag, wait_budget)) {
-        if (lane == 0) report_status(args.status, kWaitTmemEmptyTimeout, blockIdx.x, t, iter);
-        ok = false;
-        break;
-      }
-      tc_fence_after();
-      const uint32_t tmem_d = tmem_base + acc * BN;
-      const int kb0 = ks * kb_per_split;
-      const int kb1 = min(total_kb, kb0 + kb_per_split);
-      for (int kb = kb0; kb < kb1; ++kb) {
-        if (!mbar_wait(&bars->full[stage], phase, abort_flag, wait_budget)) {
-          if (lane == 0) report_status(args.status, kWaitFullTimeout, blockIdx.x, t, kb);
+    if (elect_one()) {   // one thread waits and issues
+      // ------------------------------ MMA issuer ------------------------------
+      constexpr uint32_t idesc = make_idesc(BM, BN, A_MAJOR, B_MAJOR, /*bf16*/ 1);
+      // descriptors of stage 0; the address field counts 16-byte units and stays below its 14 bits over all stages
+      const uint64_t adesc0 = A_MAJOR == 0 ? make_smem_desc(smem_u32(smem), 16, 1024) : make_smem_desc(smem_u32(smem), 8192, 1024);
+      const uint64_t bdesc0 = B_MAJOR == 0 ? make_smem_desc(smem_u32(smem) + C::kABytes, 16, 1024)
+                                           : make_smem_desc(smem_u32(smem) + C::kABytes, 8192, 1024);
+      int stage = 0;
+      uint32_t phase = 0;
+      int iter = 0;
+      bool ok = true;
+      for (int t = blockIdx.x; t < num_tiles && ok; t += gemm_ctas, ++iter) {
+        int m_blk, n_blk, ks;
+        decode_tile(t, m_blk, n_blk, ks);
+        const int acc = iter & 1;
+        const uint32_t acc_phase = (iter >> 1) & 1;
+        if (!mbar_wait(&bars->tmem_empty[acc], acc_phase ^ 1, abort_flag, wait_budget)) {
+          report_status(args.status, kWaitTmemEmptyTimeout, blockIdx.x, t, iter);
           ok = false;
           break;
         }
         tc_fence_after();
-        if (lane == 0) {
-          const uint32_t sa = smem_u32(smem + stage * C::kStageBytes);
-          const uint32_t sb = sa + C::kABytes;
-#pragma unroll
-          for (int k = 0; k < BK / 16; ++k) {
-            const uint64_t adesc = (A_MAJOR == 0) ? make_smem_desc(sa + k * 32, 16, 1024)
-                                                  : make_smem_desc(sa + k * 2048, 8192, 1024);
-            const uint64_t bdesc = (B_MAJOR == 0) ? make_smem_desc(sb + k * 32, 16, 1024)
-                                                  : make_smem_desc(sb + k * 2048, 8192, 1024);
-            umma_bf16(tmem_d, adesc, bdesc, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+        const uint32_t tmem_d = tmem_base + acc * BN;
+        const int kb0 = ks * kb_per_split;
+        const int kb1 = min(total_kb, kb0 + kb_per_split);
+        for (int kb = kb0; kb < kb1; ++kb) {
+          if (!mbar_wait(&bars->full[stage], phase, abort_flag, wait_budget)) {
+            report_status(args.status, kWaitFullTimeout, blockIdx.x, t, kb);
+            ok = false;
+            break;
           }
+          tc_fence_after();
+          const uint64_t ad = adesc0 + stage * (C::kStageBytes >> 4), bd = bdesc0 + stage * (C::kStageBytes >> 4);
+#pragma unroll
+          for (int k = 0; k < BK / 16; ++k)
+            umma_bf16(tmem_d, ad + k * ((A_MAJOR == 0 ? 32 : 2048) >> 4), bd + k * ((B_MAJOR == 0 ? 32 : 2048) >> 4), idesc,
+                      (kb > kb0 || k > 0) ? 1u : 0u);
           tc_commit(&bars->empty[stage]);  // frees the stage once these MMAs have read it
+          if (++stage == C::kStages) {
+            stage = 0;
+            phase ^= 1;
+          }
         }
-        __syncwarp();
-        if (++stage == C::kStages) {
-          stage = 0;
-          phase ^= 1;
-        }
+        if (ok) tc_commit(&bars->tmem_full[acc]);
       }
-      if (ok && lane == 0) tc_commit(&bars->tmem_full[acc]);
-      __syncwarp();
     }
   } else {
     // ------------------------------ epilogue ------------------------------

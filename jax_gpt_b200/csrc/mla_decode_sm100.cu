@@ -150,7 +150,7 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap t_pool, const __grid_const
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0 && n_it > 0) {
+    if (n_it > 0 && elect_one()) {
       bool ok = true;
       mbar_arrive_expect_tx(&sh->q_full, Cfg::kQBytes);
       for (int c = 0; c < kChunks; ++c)
@@ -200,24 +200,24 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap t_pool, const __grid_const
       }
     }
   } else if (warp == 1) {
-    // ---------------- MMA issuer (score product of tile i before the output product of tile i-1) ----------------
-    constexpr uint32_t idesc_s = make_idesc(kTile, kHeads, 0, 0, 1);
-    constexpr uint32_t idesc_pv = make_idesc(128, kHeads, 1, 0, 1);
-    const uint32_t a_kv = smem_u32(kv), a_q = smem_u32(qs), a_p = smem_u32(ps);
-    bool ok = n_it > 0;
-    if (ok && !mbar_wait(&sh->q_full, 0, abort_flag)) {
-      if (lane == 0) report_status(a.status, kWaitFullTimeout, 72, b, 0);
-      ok = false;
-    }
-    for (int it = 0; it <= n_it && ok; ++it) {
-      if (it < n_it) {
-        const int g = it & 1, u = it >> 1;
-        if (!mbar_wait(&sh->full[g], u & 1, abort_flag)) {
-          if (lane == 0) report_status(a.status, kWaitFullTimeout, 73, b, it);
-          break;
-        }
-        tc_fence_after();
-        if (lane == 0) {
+    if (elect_one()) {   // one thread waits and issues
+      // ---------------- MMA issuer (score product of tile i before the output product of tile i-1) ----------------
+      constexpr uint32_t idesc_s = make_idesc(kTile, kHeads, 0, 0, 1);
+      constexpr uint32_t idesc_pv = make_idesc(128, kHeads, 1, 0, 1);
+      const uint32_t a_kv = smem_u32(kv), a_q = smem_u32(qs), a_p = smem_u32(ps);
+      bool ok = n_it > 0;
+      if (ok && !mbar_wait(&sh->q_full, 0, abort_flag)) {
+        report_status(a.status, kWaitFullTimeout, 72, b, 0);
+        ok = false;
+      }
+      for (int it = 0; it <= n_it && ok; ++it) {
+        if (it < n_it) {
+          const int g = it & 1, u = it >> 1;
+          if (!mbar_wait(&sh->full[g], u & 1, abort_flag)) {
+            report_status(a.status, kWaitFullTimeout, 73, b, it);
+            break;
+          }
+          tc_fence_after();
           const uint32_t kvb = a_kv + g * kKvBytes;
 #pragma unroll
           for (int c = 0; c < kChunks; ++c)
@@ -227,16 +227,13 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap t_pool, const __grid_const
                         make_smem_desc(a_q + c * Cfg::kQChunkBytes + k * 32, 16, 1024), idesc_s, (c > 0 || k > 0) ? 1u : 0u);
           tc_commit(&sh->s_full[g]);
         }
-        __syncwarp();
-      }
-      if (it > 0) {
-        const int g = (it - 1) & 1, u = (it - 1) >> 1;
-        if (!mbar_wait(&sh->p_ready[g], u & 1, abort_flag)) {
-          if (lane == 0) report_status(a.status, kWaitFullTimeout, 74, b, it);
-          break;
-        }
-        tc_fence_after();
-        if (lane == 0) {
+        if (it > 0) {
+          const int g = (it - 1) & 1, u = (it - 1) >> 1;
+          if (!mbar_wait(&sh->p_ready[g], u & 1, abort_flag)) {
+            report_status(a.status, kWaitFullTimeout, 74, b, it);
+            break;
+          }
+          tc_fence_after();
           const uint32_t kvb = a_kv + g * kKvBytes;
 #pragma unroll
           for (int i = 0; i < 4; ++i)
@@ -248,7 +245,6 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap t_pool, const __grid_const
           tc_commit(&sh->kv_free[g]);
           tc_commit(&sh->pv_full[g]);
         }
-        __syncwarp();
       }
     }
   } else {

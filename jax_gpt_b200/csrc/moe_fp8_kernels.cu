@@ -217,7 +217,7 @@ ep_moe_forward_fp8_kernel(const __grid_constant__ Fp8Maps tm, const __grid_const
   const int num_tiles = alive ? tb->tile0[tb->n_slots] : 0;
   const int n1 = I / 128;
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       int ready_el = -1;
@@ -293,25 +293,25 @@ ep_moe_forward_fp8_kernel(const __grid_constant__ Fp8Maps tm, const __grid_const
       }
     }
   } else if (warp == 1) {
-    int stage = 0, iter = 0;
-    uint32_t phase = 0;
-    bool ok = true;
-    for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++iter) {
-      const TileInfo ti = decode_tile(a, tb, t);
-      if (!mbar_wait(&bars->tmem_empty, (iter & 1) ^ 1, abort_flag)) {
-        if (lane == 0) report_status(a.status, kWaitTmemEmptyTimeout, 94, blockIdx.x, t);
-        break;
-      }
-      tc_fence_after();
-      const int nslab = ti.phase == 0 ? dslabs : islabs;
-      for (int s = 0; s < nslab; ++s) {
-        if (!mbar_wait(&bars->full[stage], phase, abort_flag)) {
-          if (lane == 0) report_status(a.status, kWaitFullTimeout, 95, blockIdx.x, t);
-          ok = false;
+    if (elect_one()) {   // one thread waits and issues
+      int stage = 0, iter = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++iter) {
+        const TileInfo ti = decode_tile(a, tb, t);
+        if (!mbar_wait(&bars->tmem_empty, (iter & 1) ^ 1, abort_flag)) {
+          report_status(a.status, kWaitTmemEmptyTimeout, 94, blockIdx.x, t);
           break;
         }
         tc_fence_after();
-        if (lane == 0) {
+        const int nslab = ti.phase == 0 ? dslabs : islabs;
+        for (int s = 0; s < nslab; ++s) {
+          if (!mbar_wait(&bars->full[stage], phase, abort_flag)) {
+            report_status(a.status, kWaitFullTimeout, 95, blockIdx.x, t);
+            ok = false;
+            break;
+          }
+          tc_fence_after();
           const uint32_t sa = smem_u32(smem + stage * kStageBytes), sb = sa + kABytes;
           const uint32_t sf = smem_u32(sf_smem + stage * kStageSf);
           const uint32_t tsf = tmem_base + kSfCol0 + stage * 12;
@@ -324,15 +324,13 @@ ep_moe_forward_fp8_kernel(const __grid_constant__ Fp8Maps tm, const __grid_const
             umma_mxf8(tmem_base, make_smem_desc(sa + k * 32, 16, 1024), make_smem_desc(sb + k * 32, 16, 1024),
                       make_idesc_mx(BM, BN, k), tsf, tsf + 4, (s > 0 || k > 0) ? 1u : 0u);
           tc_commit(&bars->empty[stage]);
+          if (++stage == kStages) {
+            stage = 0;
+            phase ^= 1;
+          }
         }
-        __syncwarp();
-        if (++stage == kStages) {
-          stage = 0;
-          phase ^= 1;
-        }
+        if (ok) tc_commit(&bars->tmem_full);
       }
-      if (ok && lane == 0) tc_commit(&bars->tmem_full);
-      __syncwarp();
     }
   } else {
     // ---------------- eight epilogue warps: (lane quarter q, accumulator half) ----------------

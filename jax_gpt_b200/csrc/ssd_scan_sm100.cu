@@ -171,7 +171,7 @@ chunk_scan_kernel(const __grid_constant__ CUtensorMap t_xbc, const __grid_consta
   const uint32_t tmem = sh->tmem_base;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       const int g = h / a.rep;
       const int col_b = a.col_b + g * kN, col_c = a.col_c + g * kN, col_x = a.col_x + h * a.P + p0;
       int issued = 0;
@@ -203,64 +203,55 @@ chunk_scan_kernel(const __grid_constant__ CUtensorMap t_xbc, const __grid_consta
       }
     }
   } else if (warp == 1) {
-    constexpr uint32_t i_kk = make_idesc(128, 128, 0, 0, 1);    // G: C (K-major) x B (K-major)
-    constexpr uint32_t i_yo = make_idesc(128, 128, 0, 1, 1);    // Yo: C (K-major) x [S high | S low] (MN-major)
-    constexpr uint32_t i_y = make_idesc(128, kP, 0, 1, 1);      // Y: M (TMEM) x X (MN-major)
-    constexpr uint32_t i_t = make_idesc(128, kP, 1, 1, 1);      // T: B (MN-major) x X' (MN-major)
-    const uint32_t a_s = smem_u32(smem + kOffS), a_xp = smem_u32(smem + kOffXp);
-    auto tile = [&](int n) { return smem_u32(smem + (n & 1) * kStageBytes); };
-    auto issue_g = [&](int n) -> bool {
-      if (!mbar_wait(&sh->full[n & 1], (n >> 1) & 1, abort_flag)) {
-        if (lane == 0) report_status(a.status, kWaitFullTimeout, 311, h, n);
-        return false;
-      }
-      tc_fence_after();
-      if (lane == 0) {
+    if (elect_one()) {   // one thread waits and issues
+      constexpr uint32_t i_kk = make_idesc(128, 128, 0, 0, 1);    // G: C (K-major) x B (K-major)
+      constexpr uint32_t i_yo = make_idesc(128, 128, 0, 1, 1);    // Yo: C (K-major) x [S high | S low] (MN-major)
+      constexpr uint32_t i_y = make_idesc(128, kP, 0, 1, 1);      // Y: M (TMEM) x X (MN-major)
+      constexpr uint32_t i_t = make_idesc(128, kP, 1, 1, 1);      // T: B (MN-major) x X' (MN-major)
+      const uint32_t a_s = smem_u32(smem + kOffS), a_xp = smem_u32(smem + kOffXp);
+      auto tile = [&](int n) { return smem_u32(smem + (n & 1) * kStageBytes); };
+      auto issue_g = [&](int n) -> bool {
+        if (!mbar_wait(&sh->full[n & 1], (n >> 1) & 1, abort_flag)) {
+          report_status(a.status, kWaitFullTimeout, 311, h, n);
+          return false;
+        }
+        tc_fence_after();
         const uint32_t tc = tile(n), tb = tc + kTileBytes;
 #pragma unroll
         for (int k = 0; k < 8; ++k)   // K = state size
           umma_bf16(tmem + kColG + (n & 1) * 128, make_smem_desc(tc + (k >> 2) * 16384 + (k & 3) * 32, 16, 1024),
                     make_smem_desc(tb + (k >> 2) * 16384 + (k & 3) * 32, 16, 1024), i_kk, k > 0 ? 1u : 0u);
         tc_commit(&sh->g_full[n & 1]);
-      }
-      __syncwarp();
-      return true;
-    };
-    const bool ok = issue_g(0);
-    for (int n = 0; ok && n < n_chunks; ++n) {
-      // G(n + 1) goes into the buffer of M(n - 1), whose product Y(n - 1) was issued before and runs first
-      if (n + 1 < n_chunks && !issue_g(n + 1)) break;
-      const uint32_t tc = tile(n), tb = tc + kTileBytes, tx = tb + kTileBytes;
-      if (!mbar_wait(&sh->s_ready, n & 1, abort_flag)) {
-        if (lane == 0) report_status(a.status, kWaitFullTimeout, 312, h, n);
-        break;
-      }
-      tc_fence_after();
-      if (lane == 0) {
+        return true;
+      };
+      const bool ok = issue_g(0);
+      for (int n = 0; ok && n < n_chunks; ++n) {
+        // G(n + 1) goes into the buffer of M(n - 1), whose product Y(n - 1) was issued before and runs first
+        if (n + 1 < n_chunks && !issue_g(n + 1)) break;
+        const uint32_t tc = tile(n), tb = tc + kTileBytes, tx = tb + kTileBytes;
+        if (!mbar_wait(&sh->s_ready, n & 1, abort_flag)) {
+          report_status(a.status, kWaitFullTimeout, 312, h, n);
+          break;
+        }
+        tc_fence_after();
 #pragma unroll
         for (int k = 0; k < 8; ++k)   // K = state size; the second 64 columns are the low parts
           umma_bf16(tmem + kColYo, make_smem_desc(tc + (k >> 2) * 16384 + (k & 3) * 32, 16, 1024),
                     make_smem_desc(a_s + k * 2048, 16384, 1024), i_yo, k > 0 ? 1u : 0u);
-      }
-      __syncwarp();
-      if (!mbar_wait(&sh->m_ready[n & 1], (n >> 1) & 1, abort_flag)) {
-        if (lane == 0) report_status(a.status, kWaitFullTimeout, 313, h, n);
-        break;
-      }
-      tc_fence_after();
-      if (lane == 0) {
+        if (!mbar_wait(&sh->m_ready[n & 1], (n >> 1) & 1, abort_flag)) {
+          report_status(a.status, kWaitFullTimeout, 313, h, n);
+          break;
+        }
+        tc_fence_after();
 #pragma unroll
         for (int k = 0; k < 16; ++k)   // K = tokens; step k of M: high words at 16 k, low words at 16 k + 8
           umma_bf16_ts(tmem + kColY, tmem + kColG + (n & 1) * 128 + (k >> 1) * 16 + (k & 1) * 8,
                        make_smem_desc(tx + (k >> 1) * 2048, 16384, 1024), i_y, k > 0 ? 1u : 0u);
-      }
-      __syncwarp();
-      if (!mbar_wait(&sh->xp_ready, n & 1, abort_flag)) {
-        if (lane == 0) report_status(a.status, kWaitFullTimeout, 314, h, n);
-        break;
-      }
-      tc_fence_after();
-      if (lane == 0) {
+        if (!mbar_wait(&sh->xp_ready, n & 1, abort_flag)) {
+          report_status(a.status, kWaitFullTimeout, 314, h, n);
+          break;
+        }
+        tc_fence_after();
 #pragma unroll
         for (int k = 0; k < 16; ++k)   // K = tokens, X' high then low
           umma_bf16(tmem + kColT, make_smem_desc(tb + (k & 7) * 2048, 16384, 1024),
@@ -268,7 +259,6 @@ chunk_scan_kernel(const __grid_constant__ CUtensorMap t_xbc, const __grid_consta
         tc_commit(&sh->empty[n & 1]);
         tc_commit(&sh->y_full);
       }
-      __syncwarp();
     }
   } else if (warp < 2 + kGroup / 32) {
     // ---- chunk warps: step sizes, M, X' ----
