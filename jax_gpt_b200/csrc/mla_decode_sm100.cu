@@ -437,17 +437,30 @@ cudaError_t launch_decode_t(const CUtensorMap& t_pool, const CUtensorMap& t_q, c
 cudaError_t launch_mla_paged_decode(const __nv_bfloat16* q, const __nv_bfloat16* pool, int n_pages,
                                     const MlaDecodeArgs& args, __nv_bfloat16* out, cudaStream_t stream) {
   if (args.batch < 1 || args.heads < 1 || args.n_splits < 1 || args.max_pages < 1 || n_pages < 1) return cudaErrorInvalidValue;
+  cudaError_t e;
+  MlaDecodeArgs a2 = args;
+  a2.n_pages = n_pages;
+  if (args.heads > 64) {
+    // From 65 heads on the heads fill the 128 rows of the tensor-core tile by more than half. A key range is 2 CTAs per 128 heads:
+    // the ranges double (the scratch has room for that) where the SMs take them in one wave.
+    int dev = 0, sms = 0;
+    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+    const int64_t ctas = 2ll * args.batch * ((args.heads + 127) / 128) * args.n_splits;
+    const int n_parts = 2 * ctas <= sms ? 2 * args.n_splits : args.n_splits;
+    if ((e = launch_mla_decode_wide(q, pool, a2, n_parts, out, stream)) != cudaSuccess || n_parts == 1) return e;
+    mla_merge_kernel<<<args.batch * args.heads, kMlaLatent / 4, 0, stream>>>(args.part_out, args.part_lse, out, args.heads, n_parts,
+                                                                            args.sink);
+    return cudaGetLastError();
+  }
   const int hpc = args.heads <= 16 ? 16 : 32;   // head columns per CTA
   CUtensorMap t_pool, t_q;
-  cudaError_t e;
   if ((e = encode_tma_2d(&t_pool, pool, 2, kMlaWidth, static_cast<uint64_t>(n_pages) * kMlaPage, kMlaWidth * 2ull, 64,
                          kMlaPage)) != cudaSuccess)
     return e;
   if ((e = encode_tma_2d(&t_q, q, 2, kMlaWidth, static_cast<uint64_t>(args.batch) * args.heads, kMlaWidth * 2ull, 64,
                          hpc)) != cudaSuccess)
     return e;
-  MlaDecodeArgs a2 = args;
-  a2.n_pages = n_pages;
   e = hpc == 16 ? launch_decode_t<16>(t_pool, t_q, a2, stream) : launch_decode_t<32>(t_pool, t_q, a2, stream);
   if (e != cudaSuccess) return e;
   mla_merge_kernel<<<args.batch * args.heads, kMlaLatent / 4, 0, stream>>>(args.part_out, args.part_lse, out, args.heads,

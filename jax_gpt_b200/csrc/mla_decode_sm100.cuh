@@ -21,8 +21,8 @@ struct MlaDecodeArgs {
   const int* seq_lens;            // [max_seqs] tokens to attend over (the new token included)
   const int* seq_ids;             // [batch] row of block_table / seq_lens for every batch slot
   float scale_log2;               // softmax scale * log2(e)
-  float* part_out;                // [batch, 2 * n_splits, heads, 512] normalised partials (two softmax groups per split)
-  float* part_lse;                // [batch, 2 * n_splits, heads] log2-sum-exp of each partial (-inf when empty)
+  float* part_out;                // room for [batch, 2 * n_splits, heads, 512] normalised partials (two softmax groups per split)
+  float* part_lse;                // room for [batch, 2 * n_splits, heads] log2-sum-exps of the partials (-inf when empty)
   int* status;
   const float* sink = nullptr;    // [heads] fp32 or nullptr: exp(sink[h]) joins the softmax denominator of head h
   int window = 0;                 // > 0: only the last `window` tokens are seen
@@ -33,6 +33,11 @@ struct MlaDecodeArgs {
 // scratch: part_out / part_lse as sized above.
 cudaError_t launch_mla_paged_decode(const __nv_bfloat16* q, const __nv_bfloat16* pool, int n_pages,
                                     const MlaDecodeArgs& args, __nv_bfloat16* out, cudaStream_t stream);
+
+// The kernel for 65 and more heads (mla_decode_wide_sm100.cu): `n_parts` key ranges per sequence, at most 2 * n_splits. One range
+// writes `out`; more write [batch, n_parts, heads, 512] partials for the merge.
+cudaError_t launch_mla_decode_wide(const __nv_bfloat16* q, const __nv_bfloat16* pool, const MlaDecodeArgs& args, int n_parts,
+                                   __nv_bfloat16* out, cudaStream_t stream);
 
 // Writes rows [batch, T, width] into the pages of their sequences at positions start[b] + t.
 cudaError_t launch_paged_kv_write(const __nv_bfloat16* rows, __nv_bfloat16* pool, const int* block_table,

@@ -164,6 +164,32 @@ def test_mla_paged_decode_and_paged_write(cuda_device, heads, n_splits):
     assert rel < 1.5e-2, rel
 
 
+@pytest.mark.parametrize("heads,n_splits,window,sink", [(65, 0, 0, False), (128, 1, 0, True), (128, 3, 0, False), (128, 2, 100, True),
+                                                        (130, 0, 64, False), (256, 5, 0, True)])
+def test_mla_paged_decode_many_heads(cuda_device, heads, n_splits, window, sink):
+    """The kernel for 65 and more heads vs fp32 math: lengths around the page, more key ranges than pages, rows that grow (the
+    running maximum rises late), windows that start inside a page. The probabilities and the output are rounded to bf16, 2^-9 each;
+    both errors are independent over the tokens, so they stay near 2^-9 of the output: 1e-2 is four times their sum."""
+    from jax_gpt_b200 import _ext
+    from jax_gpt_b200.cache.paged import PagedCache
+    from jax_gpt_b200.ops.mla_decode import mla_paged_decode, mla_paged_decode_ref
+    lens = [1, 64, 65, 129, 447, 1000]
+    g = torch.Generator(device=cuda_device).manual_seed(7)
+    cache = PagedCache(1, 576, n_pages=40, page_size=64, max_seqs=8, max_pages_per_seq=20, device=cuda_device)
+    ids = [3, 0, 7, 1, 5, 2]
+    for sid, n in zip(ids, lens):
+        rows = torch.randn(1, n, 576, device=cuda_device, generator=g) * torch.linspace(0.3, 3.0, n, device=cuda_device)[None, :, None]
+        cache.append(0, [sid], rows.to(torch.bfloat16), commit=True)
+    q = torch.randn(len(lens), heads, 576, device=cuda_device, generator=g).to(torch.bfloat16)
+    sk = torch.randn(heads, device=cuda_device, generator=g) * 4 if sink else None
+    out = mla_paged_decode(q, cache, 0, ids, 192 ** -0.5, n_splits=n_splits, sink=sk, window=window)
+    torch.cuda.synchronize()
+    _ext.check_status(cuda_device)
+    ref = mla_paged_decode_ref(q.float(), cache, 0, ids, 192 ** -0.5, 512, sk, window)
+    rel = ((out.float() - ref).norm(dim=-1) / ref.norm(dim=-1)).max().item()
+    assert rel < 1e-2, rel
+
+
 @pytest.mark.parametrize("M,N,K", [(300, 512, 1024), (256, 384, 512), (1024, 2048, 7168)])
 def test_mxfp8_gemm_hardware_block_scales(cuda_device, M, N, K):
     """tcgen05 block-scaled MMA (UE8M0 scales in TMEM) vs the de-quantised fp32 product."""
