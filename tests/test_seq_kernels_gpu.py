@@ -114,6 +114,38 @@ def test_gdn_decode_step(cuda_device):
     assert _rel(state, st_ref) < 1e-4 and _rel(conv_state, cs_ref) < 1e-6
 
 
+@pytest.mark.parametrize("B,Hqk,Hv,dk,Kc,offset", [(1, 2, 2, 128, 4, 0), (5, 3, 6, 128, 4, 0), (2, 2, 16, 128, 4, 0), (1, 1, 16, 128, 4, 0),
+                                                   (2, 2, 4, 128, 3, 0), (2, 2, 4, 64, 4, 0), (2, 2, 4, 128, 4, 1)])
+def test_gdn_decode_step_routes(cuda_device, B, Hqk, Hv, dk, Kc, offset):
+    """Three steps of the register kernel (heads of 128, a window of 4, up to 8 value heads a qk head, aligned states) and of the
+    general one (16 value heads, another window or width, states one float off) vs fp32 torch. All sums are fp32: 1e-4."""
+    from jax_gpt_b200 import _ext
+    from jax_gpt_b200.models.qwen35 import deltanet as DN
+    g = torch.Generator(device=cuda_device).manual_seed(11)
+    rnd = lambda *s: torch.randn(*s, device=cuda_device, generator=g)
+    Kd, Vd = Hqk * dk, Hv * dk
+    C = 2 * Kd + Vd
+    conv_w, norm_w = (rnd(C, Kc) * 0.5).to(torch.bfloat16), (rnd(dk) * 0.3 + 1).to(torch.bfloat16)
+    A_log, dt_bias = rnd(Hv).to(torch.bfloat16), rnd(Hv).to(torch.bfloat16)
+    off = lambda t: torch.cat([t.new_zeros(offset), t.reshape(-1)])[offset:].view(t.shape)
+    conv_ref, st_ref = rnd(B, C, Kc), rnd(B, Hv, dk, dk) * 0.1
+    conv_state, state = off(conv_ref), off(st_ref)
+    for _ in range(3):
+        every = rnd(B, C + Vd + 2 * Hv).to(torch.bfloat16)               # column slices of one projection
+        mixed, z, bp, ap = every.split([C, Vd, Hv, Hv], 1)
+        mx, conv_ref = DN.causal_conv1d_update(mixed.float(), conv_ref, conv_w.float())
+        q = DN._l2_norm(mx[:, :Kd].reshape(B, Hqk, dk)) * dk ** -0.5
+        k = DN._l2_norm(mx[:, Kd:2 * Kd].reshape(B, Hqk, dk))
+        beta, gate = DN._gates(bp.float(), ap.float(), {"A_log": A_log.float(), "dt_bias": dt_bias.float()})
+        rep = lambda t: t.repeat_interleave(Hv // Hqk, 1)
+        o, st_ref = DN.gated_delta_step(rep(q), rep(k), mx[:, 2 * Kd:].reshape(B, Hv, dk), beta, gate, st_ref)
+        o = DN._gated_rms_norm(o.reshape(B * Hv, dk), z.float().reshape(B * Hv, dk), norm_w.float()).reshape(B, Vd)
+        out = torch.empty(B, Vd, device=cuda_device, dtype=torch.bfloat16)
+        _ext.ops().gdn_decode_step(mixed, z, bp, ap, conv_state, conv_w, A_log, dt_bias, norm_w, state, out, Hqk, Hv, dk, dk, 1e-6)
+        assert _rel(out, o) < 1e-2
+        assert _rel(state, st_ref) < 1e-4 and _rel(conv_state, conv_ref) < 1e-6
+
+
 @pytest.mark.parametrize("M,N,K", [(128, 128, 128), (300, 256, 512), (1024, 2048, 7168), (4096, 4096, 2048)])
 def test_fp8_blockscaled_gemm(cuda_device, M, N, K):
     from jax_gpt_b200.ops import fp8 as RP
