@@ -116,4 +116,16 @@ cudaError_t launch_gdn_conv_silu(const __nv_bfloat16* x, const __nv_bfloat16* w,
 cudaError_t launch_gdn_conv_silu_bwd(const __nv_bfloat16* x, const __nv_bfloat16* w, const __nv_bfloat16* dy,
                                      __nv_bfloat16* dx, float* dw, int B, int T, int C, int K, cudaStream_t stream);
 
+// Rotations and layouts of a prompt's latent attention (half-split pairs). rows = B * T tokens; freqs [T, dr / 2, 2] (cos, sin).
+// q [rows, H, dn + dr]: the last dr features turn in place; kvb [rows, H, dn + dv] = [key | value up-projection]; kv [rows, kvr + dr]
+// whose last dr columns are the shared key; c_kv [rows, kvr]. Writes k [rows, H, dn + dr], v [rows, H, dv], lat [rows, kvr + dr].
+cudaError_t launch_mla_prompt_rope(__nv_bfloat16* q, const __nv_bfloat16* kvb, const __nv_bfloat16* kv, const __nv_bfloat16* c_kv,
+                                   const float* freqs, __nv_bfloat16* k, __nv_bfloat16* v, __nv_bfloat16* lat, int64_t rows, int T,
+                                   int H, int dn, int dr, int dv, int kvr, cudaStream_t stream);
+// One token per sequence: q [B, H, dn + dr], q_lat [B, H, kvr] (strides lat_b, lat_h), freqs [positions, dr / 2, 2], pos [B]. Writes
+// q_full [B, H, kvr + dr] and the cache rows lat [B, kvr + dr].
+cudaError_t launch_mla_step_rope(const __nv_bfloat16* q, const __nv_bfloat16* q_lat, int64_t lat_b, int64_t lat_h,
+                                 const __nv_bfloat16* kv, const __nv_bfloat16* c_kv, const float* freqs, const int64_t* pos,
+                                 __nv_bfloat16* q_full, __nv_bfloat16* lat, int B, int H, int dn, int dr, int kvr, cudaStream_t stream);
+
 }  // namespace b200

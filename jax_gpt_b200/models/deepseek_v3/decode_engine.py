@@ -29,16 +29,6 @@ from .config import DeepSeekV3Config
 from .model import rms_norm
 
 
-def _rope_rows(x: torch.Tensor, fr: torch.Tensor) -> torch.Tensor:
-    """x (B, H, dr) or (B, dr); fr (B, dr/2, 2): every row has its own position."""
-    half = x.shape[-1] // 2
-    x1, x2 = x[..., :half].float(), x[..., half:].float()
-    cos, sin = fr[..., 0], fr[..., 1]
-    if x.dim() == 3:
-        cos, sin = cos[:, None, :], sin[:, None, :]
-    return torch.cat([x1 * cos - x2 * sin, x2 * cos + x1 * sin], dim=-1).to(x.dtype)
-
-
 class DeepSeekV3DecodeEngine:
     def __init__(self, params: dict, config: DeepSeekV3Config, cache: PagedCache, seq_ids: List[int], ep=None,
                  use_cuda_graph: bool = True, max_len: Optional[int] = None):
@@ -74,16 +64,14 @@ class DeepSeekV3DecodeEngine:
         q = linear(rms_norm(linear(x, ap["q_a_proj"]), ap["q_a_norm"], c.rms_norm_eps), ap["q_b_proj"]).reshape(B, H, dn + dr)
         kv = linear(x, ap["kv_a_proj_with_mqa"])
         c_kv = rms_norm(kv[:, :kvr].contiguous(), ap["kv_a_norm"], c.rms_norm_eps)
-        fr = self.rope.index_select(0, pos)                                   # (B, dr/2, 2)
-        q_rope = _rope_rows(q[..., dn:], fr)
-        k_rope = _rope_rows(kv[:, kvr:], fr)
         cache = self.cache
-        rows = torch.cat([c_kv, k_rope], dim=-1).to(torch.bfloat16).reshape(B, 1, kvr + dr).contiguous()
         ops = _ext.ops()
-        ops.paged_kv_write(rows, cache.pool[layer], cache.block_table, self.ids_t, pos.to(torch.int32))
         wkv = ap["kv_b_proj"].reshape(kvr, H, dn + dv)
         q_lat = torch.einsum("bhd,khd->bhk", q[..., :dn], wkv[..., :dn])
-        q_full = torch.cat([q_lat, q_rope], dim=-1).contiguous()
+        rows = torch.empty(B, 1, kvr + dr, device=x.device, dtype=torch.bfloat16)
+        q_full = torch.empty(B, H, kvr + dr, device=x.device, dtype=torch.bfloat16)
+        ops.mla_step_rope(q, q_lat, kv, c_kv, self.rope, pos, q_full, rows)
+        ops.paged_kv_write(rows, cache.pool[layer], cache.block_table, self.ids_t, pos.to(torch.int32))
         o_lat = torch.empty(B, H, 512, device=x.device, dtype=torch.bfloat16)
         # self._lens1 = lengths + 1: the token written above is attended to as well
         ops.mla_paged_decode(q_full, cache.pool[layer], cache.block_table, self._lens1, self.ids_t, c.softmax_scale,

@@ -32,6 +32,7 @@ from ...ops import attention as attn_ops
 from ...ops import grouped_gemm
 from ...ops import norm as norm_ops
 from ...ops.gemm import linear
+from ...ops.rope import mla_prompt_ok, mla_prompt_rope
 from ...utils.profiling import scope
 from ..qwen35.block import _slice
 from ..qwen35.primitives import precompute_rope_freqs
@@ -130,17 +131,24 @@ def moe_ffn(x: torch.Tensor, mp, c: DeepSeekV3Config, ep=None) -> torch.Tensor:
 
 
 # ------------------------------------------------------------------------------------------------
-def mla_project(x, ap, c: DeepSeekV3Config, rope, pos0: int):
-    """Returns q_nope (B,T,H,dn), q_rope (B,T,H,dr) rotated, c_kv (B,T,kvr) normed, k_rope (B,T,dr) rotated."""
+def _mla_down(x, ap, c: DeepSeekV3Config):
+    """q (B,T,H,dn+dr) and the latent projection kv (B,T,kvr+dr), both unrotated, and c_kv (B,T,kvr) normed."""
     B, T, _ = x.shape
-    H, dn, dr = c.n_heads, c.qk_nope_head_dim, c.qk_rope_head_dim
     q = linear(rms_norm(linear(x, ap["q_a_proj"]), ap["q_a_norm"], c.rms_norm_eps), ap["q_b_proj"])
-    q = q.reshape(B, T, H, dn + dr)
     kv = linear(x, ap["kv_a_proj_with_mqa"])
     c_kv = rms_norm(kv[..., :c.kv_lora_rank].contiguous(), ap["kv_a_norm"], c.rms_norm_eps)
-    fr = rope[pos0:pos0 + T]
+    return q.reshape(B, T, c.n_heads, c.qk_head_dim), kv, c_kv
+
+
+def mla_project(x, ap, c: DeepSeekV3Config, rope, pos0: int):
+    """Returns q_nope (B,T,H,dn), q_rope (B,T,H,dr) rotated, c_kv (B,T,kvr) normed, k_rope (B,T,dr) rotated."""
+    return _mla_rotated(*_mla_down(x, ap, c), c, rope[pos0:pos0 + x.shape[1]])
+
+
+def _mla_rotated(q, kv, c_kv, c: DeepSeekV3Config, fr):
+    dn = c.qk_nope_head_dim
     q_rope = rope_half_split(q[..., dn:], fr)
-    k_rope = rope_half_split(kv[..., c.kv_lora_rank:].reshape(B, T, 1, dr), fr)[:, :, 0]
+    k_rope = rope_half_split(kv[..., None, c.kv_lora_rank:], fr)[:, :, 0]
     return q[..., :dn], q_rope, c_kv, k_rope
 
 
@@ -148,14 +156,19 @@ def mla_prefill(x, ap, c: DeepSeekV3Config, rope, pos0: int = 0):
     """Causal MLA over the tokens of ``x`` with decompressed K/V. Returns (out (B,T,D), latent (B,T,kvr+dr))."""
     B, T, _ = x.shape
     H, dn, dr, dv = c.n_heads, c.qk_nope_head_dim, c.qk_rope_head_dim, c.v_head_dim
-    q_nope, q_rope, c_kv, k_rope = mla_project(x, ap, c, rope, pos0)
+    q, kv, c_kv = _mla_down(x, ap, c)
     kvb = linear(c_kv, ap["kv_b_proj"]).reshape(B, T, H, dn + dv)
-    k = torch.cat([kvb[..., :dn], k_rope[:, :, None, :].expand(B, T, H, dr)], dim=-1)
-    q = torch.cat([q_nope, q_rope], dim=-1)
-    v = kvb[..., dn:]
+    fr = rope[pos0:pos0 + T]
+    if mla_prompt_ok(q, kvb, kv, c_kv, fr, dv):
+        q, k, v, lat = mla_prompt_rope(q, kvb, kv, c_kv, fr, dv)
+    else:
+        q_nope, q_rope, c_kv, k_rope = _mla_rotated(q, kv, c_kv, c, fr)
+        k = torch.cat([kvb[..., :dn], k_rope[:, :, None, :].expand(B, T, H, dr)], dim=-1)
+        q = torch.cat([q_nope, q_rope], dim=-1)
+        v, lat = kvb[..., dn:], torch.cat([c_kv, k_rope], dim=-1)
     out = attn_ops.mla_attention(q, k, v, c.softmax_scale)
     y = linear(out.reshape(B, T, H * dv), ap["o_proj"])
-    return y, torch.cat([c_kv, k_rope], dim=-1)
+    return y, lat
 
 
 def mla_decode_absorbed(x, ap, c: DeepSeekV3Config, rope, cache: PagedCache, layer: int, seq_ids: List[int]):

@@ -64,6 +64,28 @@ def rmsnorm_rope(x, norm_w, freqs, rope_dim: int, pos0: int = 0, eps: float = 1e
     return y.view(B, T, H, dh)
 
 
+def mla_prompt_ok(q, kvb, kv, c_kv, freqs, dv: int) -> bool:
+    """Whether ``mla_prompt_rope`` takes these: bf16 on CUDA, contiguous on 16-byte boundaries, widths in 16-byte pieces, and nothing
+    that wants a gradient (q is turned in place)."""
+    ts = (q, kvb, kv, c_kv)
+    dr = 2 * freqs.shape[1]
+    return (all(t.is_cuda and t.dtype == torch.bfloat16 and t.is_contiguous() and t.data_ptr() % 16 == 0 for t in ts)
+            and freqs.is_cuda and freqs.dtype == torch.float32 and freqs.shape[0] == q.shape[1] and dr % 16 == 0
+            and q.shape[-1] % 8 == 0 and dv % 8 == 0 and c_kv.shape[-1] % 8 == 0
+            and not (torch.is_grad_enabled() and any(t.requires_grad for t in ts)))
+
+
+def mla_prompt_rope(q, kvb, kv, c_kv, freqs, dv: int):
+    """q (B,T,H,dn+dr), turned in place; kvb (B,T,H,dn+dv) = [key | value up-projection]; kv (B,T,kvr+dr) whose last dr features are
+    the shared key; c_kv (B,T,kvr); freqs (T,dr/2,2), half-split pairs. Returns q, k (B,T,H,dn+dr), v (B,T,H,dv) and the cache rows
+    (B,T,kvr+dr), in one launch."""
+    k = torch.empty_like(q)
+    v = torch.empty(*q.shape[:3], dv, device=q.device, dtype=q.dtype)
+    lat = torch.empty_like(kv)
+    _ext.ops().mla_prompt_rope(q, kvb, kv, c_kv, freqs.contiguous(), k, v, lat)
+    return q, k, v, lat
+
+
 # ---- interleaved rotation with optional YaRN scaling ---------------------------------------------------------------
 def yarn_frequencies(dims: int, base: float, scaling=None):
     """(frequencies [dims / 2] as Python floats, factor of cos and sin). ``scaling`` is None or a mapping with

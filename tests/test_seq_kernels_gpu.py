@@ -222,6 +222,37 @@ def test_mla_paged_decode_many_heads(cuda_device, heads, n_splits, window, sink)
     assert rel < 1e-2, rel
 
 
+@pytest.mark.parametrize("B,T,H,dn,dr,dv,kvr", [(2, 5, 3, 128, 64, 128, 512), (1, 1, 1, 8, 16, 8, 8), (1, 300, 128, 128, 64, 128, 512)])
+def test_mla_rope_layout_kernels(cuda_device, B, T, H, dn, dr, dv, kvr):
+    """Prompt and step forms vs the slices, rotations and concatenations they stand for. Copies are exact; a rotated value is one fp32
+    product sum rounded to bf16, so the two differ by a bf16 step (2^-8) at most where a contraction moves the rounding."""
+    from jax_gpt_b200 import _ext
+    from jax_gpt_b200.models.deepseek_v3.model import rope_half_split
+    from jax_gpt_b200.models.qwen35.primitives import precompute_rope_freqs
+    from jax_gpt_b200.ops import rope as R
+    g = torch.Generator(device=cuda_device).manual_seed(3)
+    bf = lambda *s: torch.randn(*s, device=cuda_device, generator=g).to(torch.bfloat16)
+    q, kvb, kv, c_kv = bf(B, T, H, dn + dr), bf(B, T, H, dn + dv), bf(B, T, kvr + dr), bf(B, T, kvr)
+    table = precompute_rope_freqs(dr, T + 40, 10000.0, device=cuda_device)
+    near = lambda a, b: torch.equal(a[..., :-dr], b[..., :-dr]) and torch.allclose(a.float(), b.float(), rtol=2 ** -7, atol=1e-6)
+    fr = table[7:7 + T]
+    qr, kr = rope_half_split(q[..., dn:], fr), rope_half_split(kv[..., None, kvr:], fr)
+    assert R.mla_prompt_ok(q, kvb, kv, c_kv, fr, dv) and not R.mla_prompt_ok(q.clone().requires_grad_(), kvb, kv, c_kv, fr, dv)
+    want_q = torch.cat([q[..., :dn], qr], -1)
+    q2, k, v, lat = R.mla_prompt_rope(q.clone(), kvb, kv, c_kv, fr, dv)
+    assert near(q2, want_q) and near(k, torch.cat([kvb[..., :dn], kr.expand(B, T, H, dr)], -1))
+    assert torch.equal(v, kvb[..., dn:]) and near(lat, torch.cat([c_kv, kr[:, :, 0]], -1))
+    # the step form: B * T sequences of one token, positions of their own, q_lat head-major as the batched product leaves it
+    n = B * T
+    pos = torch.randint(0, T + 40, (n,), device=cuda_device, generator=g)
+    q_lat = bf(H, n, kvr).transpose(0, 1)
+    q_full, rows = torch.empty(n, H, kvr + dr, device=cuda_device, dtype=torch.bfloat16), torch.empty(n, kvr + dr, device=cuda_device, dtype=torch.bfloat16)
+    _ext.ops().mla_step_rope(q.view(n, H, dn + dr), q_lat, kv.view(n, -1), c_kv.view(n, -1), table, pos, q_full, rows)
+    turn = lambda x: rope_half_split(x.reshape(1, n, -1, dr), table[pos])[0]
+    assert near(q_full, torch.cat([q_lat, turn(q.view(n, H, -1)[..., dn:])], -1))
+    assert near(rows, torch.cat([c_kv.view(n, -1), turn(kv.view(n, -1)[:, kvr:])[:, 0]], -1))
+
+
 @pytest.mark.parametrize("M,N,K", [(300, 512, 1024), (256, 384, 512), (1024, 2048, 7168)])
 def test_mxfp8_gemm_hardware_block_scales(cuda_device, M, N, K):
     """tcgen05 block-scaled MMA (UE8M0 scales in TMEM) vs the de-quantised fp32 product."""
