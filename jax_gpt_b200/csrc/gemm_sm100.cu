@@ -177,6 +177,20 @@ __device__ void stage_copier_ldst(const StageCopy& sc, int idx, int n_workers) {
   }
 }
 
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t cluster_address(uint32_t saddr, int rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ float cluster_load_f32(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+  return v;
+}
+
 template <int BN, int A_MAJOR, int B_MAJOR>
 __global__ void __launch_bounds__(kNumThreads, 1)
 gemm_bf16_kernel(const __grid_constant__ TmaSet tma_a, const __grid_constant__ TmaSet tma_b,
@@ -200,7 +214,8 @@ gemm_bf16_kernel(const __grid_constant__ TmaSet tma_a, const __grid_constant__ T
 
   const int m_blocks = (args.M + BM - 1) / BM;
   const int n_blocks = (args.N + BN - 1) / BN;
-  const int split_k = args.split_k < 1 ? 1 : args.split_k;
+  const int cluster_k = args.cluster_k < 1 ? 1 : args.cluster_k;     // the CTAs of a cluster share a tile's K range
+  const int split_k = cluster_k > 1 ? cluster_k : (args.split_k < 1 ? 1 : args.split_k);
   const int total_kb = (args.K + BK - 1) / BK;
   const int kb_per_split = (total_kb + split_k - 1) / split_k;
   const int num_tiles = m_blocks * n_blocks * split_k;
@@ -433,6 +448,21 @@ gemm_bf16_kernel(const __grid_constant__ TmaSet tma_a, const __grid_constant__ T
         break;
       }
       tc_fence_after();
+      if (cluster_k > 1) {
+        // one tile per CTA: the partial sums go where the operands were (all of them have been read), column by column
+        if (m_blk * BM + q * 32 < args.M) {
+          float* part = reinterpret_cast<float*>(smem);
+#pragma unroll 1
+          for (int c = half * (BN / 2); c < (half + 1) * (BN / 2); c += 32) {
+            uint32_t v[32];
+            tmem_ld_32x32(tmem_base + acc * BN + (static_cast<uint32_t>(q * 32) << 16) + c, v);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 32; ++j) part[(c + j) * BM + q * 32 + lane] = __uint_as_float(v[j]);
+          }
+        }
+        break;
+      }
       // Empty K range (possible only for trailing splits): nothing was accumulated.
       const bool has_k = ks * kb_per_split < total_kb;
       gemm_epilogue_columns(args, tmem_base + acc * BN + (static_cast<uint32_t>(q * 32) << 16),
@@ -460,6 +490,31 @@ gemm_bf16_kernel(const __grid_constant__ TmaSet tma_a, const __grid_constant__ T
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, C::kTmemCols);
+  }
+  if (cluster_k > 1) {
+    // Sum of the cluster's partial tiles, in the order of the K ranges, by the CTA that owns the columns; every thread of every CTA
+    // gets here, also after a wait that gave up.
+    cluster_barrier();
+    int m_blk, n_blk, ks;
+    decode_tile(blockIdx.x, m_blk, n_blk, ks);
+    const int q = warp & 3, half = (warp - 2) >> 2, per = BN / cluster_k;     // 64 or 32 columns per CTA, 32 per warp
+    const int c = ks * per + half * 32, row0 = m_blk * BM + q * 32;
+    if (warp >= 2 && half * 32 < per && row0 < args.M && n_blk * BN + c < args.N) {
+      const uint32_t mine = smem_u32(smem) + (c * BM + q * 32 + lane) * 4;
+      float sum[32];
+#pragma unroll
+      for (int j = 0; j < 32; ++j) sum[j] = 0.f;
+      for (int p = 0; p < cluster_k; ++p) {
+        const uint32_t at = cluster_address(mine, p);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) sum[j] += cluster_load_f32(at + j * BM * 4);
+      }
+      uint32_t v[32];
+#pragma unroll
+      for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(sum[j]);
+      if (row0 + lane < args.M) gemm_epilogue_chunk(args, v, row0 + lane, n_blk * BN + c, 0);
+    }
+    cluster_barrier();     // nobody leaves while its shared memory is being read
   }
   if (args.out_mode == kOutBf16PeerPush) {
     // second phase of GEMM -> reduce-scatter: sum the n_peers bf16 partials of this rank's rows. A unit is one
@@ -511,6 +566,20 @@ cudaError_t launch_variant(const TmaSet& ta, const TmaSet& tb, const GemmArgs& a
   }
   const int m_blocks = (args.M + BM - 1) / BM;
   const int n_blocks = (args.N + BN - 1) / BN;
+  if (args.cluster_k > 1) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(m_blocks * n_blocks * args.cluster_k);
+    cfg.blockDim = dim3(kNumThreads);
+    cfg.dynamicSmemBytes = C::kSmemBytes;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = args.cluster_k;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, ta, tb, args, gi, sc);
+  }
   const int tiles = m_blocks * n_blocks * (args.split_k < 1 ? 1 : args.split_k);
   // copier CTAs must be resident together with the compute CTAs that wait for them: the grid never exceeds the
   // SM count (one CTA per SM by shared memory)
@@ -526,6 +595,18 @@ cudaError_t make_operand_map(CUtensorMap* map, const __nv_bfloat16* p, int64_t l
   // K-major: stored [rows_mn, K], box {64 (k), box_mn}. MN-major: stored [K, rows_mn], box {64 (mn), 64 (k)}.
   if (major == 0) return encode_tma_2d(map, p, /*elem*/ 2, /*inner*/ K, /*outer*/ rows_mn, ld * 2, 64, box_mn);
   return encode_tma_2d(map, p, 2, rows_mn, K, ld * 2, 64, 64);
+}
+
+// CTAs that share the K range of a 128 x 128 tile where the tiles leave SMs idle. A 64-deep k-block takes 0.16 us, handing the partial
+// sums round through the cluster's shared memory 2 - 3 us: four CTAs win from 32 k-blocks on, two from 48. One CTA, then as chosen here,
+// for rows x out x in: 1 x 512 x 2048 10.0 -> 8.4 us (four), 1 x 2048 x 4096 16.4 -> 12.1 (four), 64 x 1536 x 7168 24.2 -> 14.8 (four),
+// 64 x 7168 x 18432 50 -> 47 (two); 768 x 768 x 999 lost 1.2 us on two CTAs. Pairs fit the SMs exactly; clusters of four leave some of a
+// GPC's SMs over, so only as many as surely run in one wave. No K range is empty. The sums are fp32 in a fixed order.
+int cluster_split(int tiles, int k_blocks) {
+  const int sms = gemm_sm_count();
+  if (k_blocks >= 32 && 4 * tiles <= sms - 16) return 4;
+  if (k_blocks >= 48 && 2 * tiles <= sms) return 2;
+  return 1;
 }
 
 cudaError_t launch_common(const __nv_bfloat16* const* a_src, int n_src, int rows_per_src, int first_src, int64_t lda,
@@ -550,6 +631,9 @@ cudaError_t launch_common(const __nv_bfloat16* const* a_src, int n_src, int rows
                                         gemm_sm_count());
   int BN = wide ? 256 : 128;
   if (b_n_src > 1 && (args.N / b_n_src) % BN != 0) BN = 128;     // a tile must not straddle two weight shards
+  args.cluster_k = 1;
+  if (n_src == 1 && b_n_src == 1 && stage_copy == nullptr && BN == 128 && args.split_k == 0 && args.out_mode <= kOutF32Atomic)
+    args.cluster_k = cluster_split(m_blocks * ((args.N + BN - 1) / BN), (args.K + BK - 1) / BK);
 
   TmaSet ta;
   for (int s = 0; s < n_src; ++s) {

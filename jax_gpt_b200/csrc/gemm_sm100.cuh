@@ -41,7 +41,8 @@ struct GemmArgs {
   int out_mode;
   float alpha;
   float act_a, act_b;             // kEpiXielu
-  int split_k;
+  int split_k;                    // > 1: K ranges as tiles of their own (fp32 atomics); 1: one CTA sums a tile; 0: the launcher chooses
+  int cluster_k;                  // set by the launcher: CTAs of a cluster that share a tile's K range and sum on chip
   int* status;
   // kOutBf16PeerRed: rows [r*rows_per_peer, (r+1)*rows_per_peer) of the logical output live
   // in peer_out[r] (this rank's own buffer included), each [rows_per_peer, ldo] fp32.

@@ -73,7 +73,9 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn_major: bool = False, b_mn_maj
          residual: Optional[torch.Tensor] = None, aux: Optional[torch.Tensor] = None, epilogue: int = EPI_NONE,
          out_mode: int = OUT_BF16, alpha: float = 1.0, split_k: int = 1, act_args=(0.0, 0.0)) -> torch.Tensor:
     """See module docstring. ``out_mode=OUT_F32_ATOMIC`` accumulates into ``out`` (fp32). ``act_args``: the two constants of
-    ``EPI_XIELU``."""
+    ``EPI_XIELU``. ``split_k`` > 1 (with fp32 accumulation) adds up that many K ranges by atomics; 0 lets the launcher share the K range
+    of few tiles among CTAs, with another (fixed) order of sums. The GPT-2 engine keeps 1: behind AdamW's normalisation a bias whose true
+    gradient is zero, as the keys' is, moves by the sign of rounding errors, and another order would give other weights."""
     if not a.is_cuda:
         return gemm_ref(a, b, a_mn_major=a_mn_major, b_mn_major=b_mn_major, out=out, bias=bias, residual=residual,
                         aux=aux, epilogue=epilogue, out_mode=out_mode, alpha=alpha, split_k=split_k, act_args=act_args)
@@ -107,7 +109,7 @@ class _LinearF32OutFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w):
         x2 = x.reshape(-1, x.shape[-1])
-        y = gemm(x2, w, b_mn_major=True, out_mode=OUT_F32)
+        y = gemm(x2, w, b_mn_major=True, out_mode=OUT_F32, split_k=0)
         ctx.save_for_backward(x2, w)
         ctx.xshape = x.shape
         return y.reshape(*x.shape[:-1], w.shape[1])
@@ -159,7 +161,7 @@ def linear_rows(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = 
             x = x.contiguous()
         if act is None or mode == 0:
             return gemm(x, w, out=out, epilogue=_ROW_ACTS[act][1],
-                        out_mode=(OUT_BF16, OUT_F32, OUT_F32_ATOMIC)[mode], act_args=act_args)
+                        out_mode=(OUT_BF16, OUT_F32, OUT_F32_ATOMIC)[mode], act_args=act_args, split_k=0)
     y = x @ w.t() if mode == 0 else x.float() @ w.float().t()
     if act == "relu2":
         y = y.clamp_min(0).square()
@@ -204,7 +206,7 @@ class _LinearFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w, bias):
         x2 = x.reshape(-1, x.shape[-1])
-        y = gemm(x2, w, b_mn_major=True, bias=bias)
+        y = gemm(x2, w, b_mn_major=True, bias=bias, split_k=0)
         ctx.save_for_backward(x2, w)
         ctx.has_bias = bias is not None
         ctx.xshape = x.shape

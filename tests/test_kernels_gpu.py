@@ -26,6 +26,30 @@ def test_gemm_layouts(cuda_device, M, N, K, a_mn, b_mn):
     assert _rel_err(out, ref) < 1e-2
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 512, 2048), (33, 136, 2120), (129, 768, 3072), (999, 768, 3080), (256, 1024, 1160), (40, 4096, 2400)])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, True), (False, False), (True, True)])
+def test_gemm_few_tiles_share_their_k_range(cuda_device, M, N, K, a_mn, b_mn):
+    """Few 128 x 128 tiles over a long K: clusters of two or four CTAs sum a tile. Rows and columns past the end, K ranges of unlike
+    length, every output mode and epilogue. K fp32 additions are off by K 2^-24 at most (2e-4), a bf16 result by 2^-9 more."""
+    from jax_gpt_b200.ops import gemm as G
+    if a_mn and M % 8:
+        pytest.skip("row strides must be multiples of 8 elements")
+    g = torch.Generator(device=cuda_device).manual_seed(2)
+    rnd = lambda *s: torch.randn(*s, device=cuda_device, generator=g).to(torch.bfloat16)
+    a, b = rnd(*((K, M) if a_mn else (M, K))), rnd(*((K, N) if b_mn else (N, K)))
+    ref = (a.double().t() if a_mn else a.double()) @ (b.double() if b_mn else b.double().t())
+    kw = dict(a_mn_major=a_mn, b_mn_major=b_mn, split_k=0)
+    assert _rel_err(G.gemm(a, b, out_mode=G.OUT_F32, **kw), ref) < 2e-4
+    acc = torch.full((M, N), 3.0, device=cuda_device)
+    assert _rel_err(G.gemm(a, b, out=acc, out_mode=G.OUT_F32_ATOMIC, **kw), ref + 3.0) < 2e-4
+    bias, res = rnd(N), rnd(M, N)
+    assert _rel_err(G.gemm(a, b, bias=bias, residual=res, **kw), ref + bias.double() + res.double()) < 4e-3
+    aux, scale = torch.empty(M, N, device=cuda_device, dtype=torch.bfloat16), 0.05
+    out = G.gemm(a, b, bias=bias, aux=aux, epilogue=G.EPI_GELU, alpha=scale, **kw)
+    assert _rel_err(aux, ref * scale + bias.double()) < 4e-3
+    assert _rel_err(out, G.gelu_tanh(aux.double())) < 4e-3      # of the rounded pre-activation
+
+
 def test_gemm_epilogues(cuda_device):
     from jax_gpt_b200.ops import gemm as G
     torch.manual_seed(1)
