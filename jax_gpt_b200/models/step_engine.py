@@ -21,7 +21,7 @@ from typing import Dict, Hashable, List, Optional, Sequence
 import torch
 
 from ..cache.hybrid import HybridPagedCache
-from ..ops.packed import PackedBatch
+from ..ops.packed import PackedBatch, upload
 
 
 class _DecodeSlot:
@@ -96,7 +96,7 @@ class StepEngine:
                     self.release(s)
             raise
         batch = PackedBatch.make(slots, lens, not any(starts), max(s + n for s, n in zip(starts, lens)), self.device)
-        tok = torch.tensor(flat, dtype=torch.int32).to(self.device)
+        tok = upload(flat, torch.int32, self.device)
         x = self.run_layers(self.params, c, self.cache, batch, tok, self.rope, layers_out)
         paged.end_step(slots, lens)
         rows, c0 = [], 0
@@ -106,7 +106,7 @@ class StepEngine:
         if not rows:
             return None
         if len(rows) != x.shape[0] or rows != list(range(len(rows))):
-            x = x[torch.tensor(rows, device=self.device)]
+            x = x[upload(rows, torch.long, self.device)]
         return self.output_logits(self.params, c, x)
 
     @torch.no_grad()

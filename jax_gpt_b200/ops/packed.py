@@ -16,6 +16,13 @@ from .. import _ext
 from .norm import LAYERNORM, RMSNORM, norm_ref
 
 
+def upload(values, dtype, device) -> torch.Tensor:
+    """A host list as a tensor on ``device``. To CUDA through page-locked memory without waiting: a plain copy would hold the host
+    until the stream is idle, so that the GPU runs dry while the next launches are prepared."""
+    t = torch.tensor(values, dtype=dtype)
+    return t.pin_memory().to(device, non_blocking=True) if torch.device(device).type == "cuda" else t.to(device)
+
+
 @dataclass
 class PackedBatch:
     seq_ids: List[int]                 # cache slots (host)
@@ -53,8 +60,7 @@ class PackedBatch:
         for n in lens:
             cu.append(cu[-1] + n)
         tok = [b for b, n in enumerate(lens) for _ in range(n)]
-        host = torch.tensor(list(seq_ids) + cu + tok, dtype=torch.int32)
-        dev = host.to(device)          # one upload
+        dev = upload(list(seq_ids) + cu + tok, torch.int32, device)
         z = torch.zeros(2, B, dtype=torch.int32, device=device)
         return PackedBatch(list(seq_ids), list(lens), fresh, max_len, dev[:B].clone(), dev[B:2 * B + 1].clone(),
                            dev[2 * B + 1:2 * B + 1 + N].clone(), z[0].clone(), z[1].clone())

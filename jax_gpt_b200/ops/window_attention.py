@@ -16,7 +16,7 @@ import torch
 
 from .. import _ext
 from . import attention as A
-from .packed import PackedBatch
+from .packed import PackedBatch, upload
 from .rope import rotate_half_split
 
 TENSOR_WIDTHS = (64, 128, 256)
@@ -127,7 +127,7 @@ def pool_layout(batch: PackedBatch, window: int, pool: int) -> PoolLayout:
         for p, n in zip(pads, batch.lens):
             firsts.append(at + p)
             at += p + n
-        dev = torch.tensor([firsts, pads], dtype=torch.int32).to(batch.ids.device)
+        dev = upload([firsts, pads], torch.int32, batch.ids.device)
         return PoolLayout(pads, at, dev[0], dev[1])
     return batch.memo(("pool_layout", window, pool), make)
 
