@@ -181,84 +181,294 @@ struct PrepFwdArgs {
   PrepGeom gm;
 };
 
-constexpr int kFwdSmemFloats = 2 * kC * kLd + kC * kC + 8 * kC;
+// ---- forward -----------------------------------------------------------------------------------------------------------
+// Bound by instruction issue, not by bytes (0.2 GB for 4096 tokens and 32 heads): with a right-hand side column per thread and the
+// substitution unrolled over 64 registers the kernel ran at a fifth of the issue rate, its 43 KB of straight-line code and the
+// chain through every row of the substitution exposed at two CTAs per SM. The products are matrix instructions here:
+//   - the Gram matrices from the raw bf16 rows, whose products are exact; the norms scale the fp32 sums;
+//   - T = (I + A)^-1 in fp32: the four 16 x 16 blocks on the diagonal by substitution, a column per thread, then two doublings
+//     T21 = -T22 (A21 T11), each two small products over the whole block;
+//   - X = (T diag(beta)) V and (T diag(beta exp(G) / |k|)) K: again raw bf16 rows on the right; the fp32 factor on the left is cut
+//     into three bf16 parts (24 bits), so nothing is rounded that was not before.
+// 4096 tokens, 32 value heads: 349 -> 131 us; against 64 bits the outputs are off by the same 1.66e-3 (their rounding to bf16).
+constexpr int kRawLd = kD + 8;    // row stride (bf16) of the raw tiles: eight rows of 16 bytes fall into different banks
+constexpr int kALd = kC + 4;      // row stride (floats) of A
+constexpr int kTLd = kC + 8;      // and of T, which is read as pairs of floats of eight rows
+constexpr int kULd = 32 + 4;
 
-__global__ void __launch_bounds__(kThreads) gdn_chunk_prep_fwd_kernel(const PrepFwdArgs p) {
-  extern __shared__ __align__(16) float smem[];
-  float* sq = smem;
-  float* sk = sq + kC * kLd;
-  float* sA = sk + kC * kLd;
-  float* s_beta = sA + kC * kC;
-  float* s_g = s_beta + kC;
-  float* s_G = s_g + kC;
-  float* s_eg = s_G + kC;
-  float* s_ed = s_eg + kC;
-  float* s_asig = s_ed + kC;
-  float* s_rq = s_asig + kC;
-  float* s_rk = s_rq + kC;
+struct PrepFwdSmem {
+  __nv_bfloat16 q[kC * kRawLd], k[kC * kRawLd], v[kC * kRawLd];
+  float A[kC * kALd], T[kC * kTLd], U[32 * kULd];
+  float beta[kC], G[kC], eg[kC], ed[kC], rq[kC], rk[kC], kscale[kC];
+  float warp0_sum;
+};
+
+__device__ __forceinline__ void mma_16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], const void* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(p)) : "memory");
+}
+__device__ __forceinline__ void ldsm4_t(uint32_t (&r)[4], const void* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(p)) : "memory");
+}
+
+// 64 rows of 128 features from column `col` of the projections, zeros from row T on.
+__device__ __forceinline__ void load_raw_tile(const __nv_bfloat16* mixed_b, const PrepGeom& gm, int n, int col, __nv_bfloat16* dst) {
+#pragma unroll
+  for (int i = threadIdx.x; i < kC * (kD / 8); i += kThreads) {
+    const int r = i >> 4, c8 = i & 15, t = n * kC + r;
+    uint4 u = make_uint4(0, 0, 0, 0);
+    if (t < gm.T) u = *reinterpret_cast<const uint4*>(mixed_b + static_cast<size_t>(t) * gm.conv_dim + col + c8 * 8);
+    *reinterpret_cast<uint4*>(dst + r * kRawLd + c8 * 8) = u;
+  }
+}
+
+// out (rows x cols) = sign * a (rows x inner) b (inner x cols), fp32 in shared memory, a thread per output, rows * cols a multiple
+// of the block; `blocks` such products, the operands a step apart.
+template <int kRows, int kCols, int kInner>
+__device__ __forceinline__ void small_product(float* out, int ldo, const float* a, int lda, const float* b, int ldb, float sign,
+                                              int blocks, int out_step, int a_step, int b_step) {
+  const int per = kRows * kCols;
+  for (int o = threadIdx.x; o < blocks * per; o += kThreads) {
+    const int blk = o / per, r = (o % per) / kCols, c = o % kCols;
+    const float* ar = a + blk * a_step + r * lda;
+    const float* bc = b + blk * b_step + c;
+    float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+#pragma unroll
+    for (int m = 0; m < kInner; m += 4) {
+      const float4 x = *reinterpret_cast<const float4*>(ar + m);
+      s0 = fmaf(x.x, bc[m * ldb], s0);
+      s1 = fmaf(x.y, bc[(m + 1) * ldb], s1);
+      s2 = fmaf(x.z, bc[(m + 2) * ldb], s2);
+      s3 = fmaf(x.w, bc[(m + 3) * ldb], s3);
+    }
+    out[blk * out_step + r * ldo + c] = sign * ((s0 + s1) + (s2 + s3));
+  }
+}
+
+// T = (I + A)^-1 of the strictly lower triangular A; blocks of T above the diagonal that a product reads are cleared.
+__device__ __forceinline__ void unit_lower_inverse(const float* A, float* T, float* U) {
+  const int tid = threadIdx.x;
+  if (tid < kC) {
+    const int b0 = tid & ~15, j = tid & 15;
+    float x[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      float acc[4] = {i == j ? 1.f : 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int m = 0; m < i; ++m) acc[m & 3] = fmaf(-A[(b0 + i) * kALd + b0 + m], x[m], acc[m & 3]);
+      x[i] = (acc[0] + acc[1]) + (acc[2] + acc[3]);
+      T[(b0 + i) * kTLd + tid] = x[i];
+    }
+  } else if (tid >= 128) {
+    for (int i = tid - 128; i < 512; i += 128) {   // the blocks right of the first and of the third on the diagonal
+      const int r = (i >> 8) * 32 + ((i >> 4) & 15), c = (i >> 8) * 32 + 16 + (i & 15);
+      T[r * kTLd + c] = 0.f;
+    }
+  }
+  __syncthreads();
+  small_product<16, 16, 16>(U, kULd, A + 16 * kALd, kALd, T, kTLd, 1.f, 2, 16 * kULd, 32 * kALd + 32, 32 * kTLd + 32);
+  __syncthreads();
+  small_product<16, 16, 16>(T + 16 * kTLd, kTLd, T + 16 * kTLd + 16, kTLd, U, kULd, -1.f, 2, 32 * kTLd + 32, 32 * kTLd + 32, 16 * kULd);
+  __syncthreads();
+  small_product<32, 32, 32>(U, kULd, A + 32 * kALd, kALd, T, kTLd, 1.f, 1, 0, 0, 0);
+  __syncthreads();
+  small_product<32, 32, 32>(T + 32 * kTLd, kTLd, T + 32 * kTLd + 32, kTLd, U, kULd, -1.f, 1, 0, 0, 0);
+  __syncthreads();
+}
+
+__global__ void __launch_bounds__(kThreads, 2) gdn_chunk_prep_fwd_kernel(const PrepFwdArgs p) {
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  PrepFwdSmem& sm = *reinterpret_cast<PrepFwdSmem*>(smem_raw);
   const PrepGeom gm = p.gm;
-  const int tid = threadIdx.x, n = blockIdx.x, hq = blockIdx.y, batch = blockIdx.z;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
+  const int n = blockIdx.x, hq = blockIdx.y, batch = blockIdx.z;
   const int rep = gm.Hv / gm.Hqk;
   const __nv_bfloat16* mixed_b = p.mixed + static_cast<size_t>(batch) * gm.T * gm.conv_dim;
-  load_qk_normalised(mixed_b, gm, n, hq, sq, sk, s_rq, s_rk);
-  const int ti = tid >> 4, tj = tid & 15;
-  float s[4][4], w[4][4];
-  gram_blocks(sq, sk, ti, tj, s, w);
+  load_raw_tile(mixed_b, gm, n, hq * kD, sm.q);
+  load_raw_tile(mixed_b, gm, n, gm.Hqk * kD + hq * kD, sm.k);
+  __syncthreads();
+  {
+    // reciprocal norms, four threads per row
+    const int i = tid >> 2, qd = tid & 3;
+    float ssq = 0.f, ssk = 0.f;
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      const uint4 a = *reinterpret_cast<const uint4*>(sm.q + i * kRawLd + (qd + 4 * m) * 8);
+      const uint4 b = *reinterpret_cast<const uint4*>(sm.k + i * kRawLd + (qd + 4 * m) * 8);
+      const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, bw[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 x = unpack_bf16x2(aw[e]), y = unpack_bf16x2(bw[e]);
+        ssq += x.x * x.x + x.y * x.y;
+        ssk += y.x * y.x + y.y * y.y;
+      }
+    }
+    ssq += __shfl_xor_sync(0xffffffffu, ssq, 1);
+    ssq += __shfl_xor_sync(0xffffffffu, ssq, 2);
+    ssk += __shfl_xor_sync(0xffffffffu, ssk, 1);
+    ssk += __shfl_xor_sync(0xffffffffu, ssk, 2);
+    if (qd == 0) {
+      sm.rq[i] = rsqrtf(ssq + 1e-6f) * kQScale;
+      sm.rk[i] = rsqrtf(ssk + 1e-6f);
+    }
+  }
+  __syncthreads();
+  // Gram matrices: warps 0-3 the row tiles of k^ k^T, warps 4-7 those of q^ k^T; entries above the diagonal are not computed
+  const int mt = warp & 3, row_lo = mt * 16 + g, row_hi = row_lo + 8;
+  const bool of_q = warp >= 4;
+  float gram[8][4];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) gram[j][0] = gram[j][1] = gram[j][2] = gram[j][3] = 0.f;
+  {
+    const __nv_bfloat16* left = of_q ? sm.q : sm.k;
+#pragma unroll
+    for (int ks = 0; ks < kD / 16; ++ks) {
+      uint32_t a[4];
+      ldsm4(a, left + (mt * 16 + (lane & 15)) * kRawLd + ks * 16 + (lane >> 4) * 8);
+#pragma unroll
+      for (int j2 = 0; j2 < 4; ++j2) {
+        if (j2 > mt) continue;
+        uint32_t b[4];
+        ldsm4(b, sm.k + (j2 * 16 + (lane >> 4) * 8 + (lane & 7)) * kRawLd + ks * 16 + ((lane >> 3) & 1) * 8);
+        mma_16816(gram[2 * j2], a, b[0], b[1]);
+        mma_16816(gram[2 * j2 + 1], a, b[2], b[3]);
+      }
+    }
+    const float* rl = of_q ? sm.rq : sm.rk;
+    const float lo = rl[row_lo], hi = rl[row_hi];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float c0 = sm.rk[j * 8 + 2 * t4], c1 = sm.rk[j * 8 + 2 * t4 + 1];
+      gram[j][0] *= lo * c0;
+      gram[j][1] *= lo * c1;
+      gram[j][2] *= hi * c0;
+      gram[j][3] *= hi * c1;
+    }
+  }
+
   for (int r = 0; r < rep; ++r) {
     const int hv = hq * rep + r;
     const size_t chunk = (static_cast<size_t>(batch) * gm.Hv + hv) * gm.N + n;
-    chunk_gates(p.b_in, p.a_in, -expf(p.A_log[hv]), p.dt_bias[hv], gm, batch, n, hv, s_beta, s_g, s_G, s_eg, s_ed, s_asig);
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int b = 0; b < 4; ++b) {
-        const int i = ti + 16 * a, j = tj + 16 * b;
-        const float D = j <= i ? expf(s_G[i] - s_G[j]) : 0.f;
-        sA[i * kC + j] = j < i ? s_beta[i] * s[a][b] * D : 0.f;
-        p.intra[(chunk * kC + i) * kC + j] = __float2bfloat16(j <= i ? w[a][b] * D : 0.f);
+    load_raw_tile(mixed_b, gm, n, 2 * gm.Hqk * kD + hv * kD, sm.v);
+    // gates (see chunk_gates), the cumulative sum by two warps
+    float beta = 0.f, G = 0.f;
+    if (tid < kC) {
+      const int t = n * kC + tid;
+      if (t < gm.T) {
+        const size_t off = (static_cast<size_t>(batch) * gm.T + t) * gm.Hv + hv;
+        beta = sigmoid_f(bf2f(p.b_in + off));
+        G = -expf(p.A_log[hv]) * softplus_f(bf2f(p.a_in + off) + p.dt_bias[hv]);
       }
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const float up = __shfl_up_sync(0xffffffffu, G, o);
+        if (lane >= o) G += up;
+      }
+      if (tid == 31) sm.warp0_sum = G;
+    }
     __syncthreads();
+    if (tid < kC) {
+      if (tid >= 32) G += sm.warp0_sum;
+      const float eg = expf(G);
+      sm.beta[tid] = beta;
+      sm.G[tid] = G;
+      sm.eg[tid] = eg;
+      sm.kscale[tid] = beta * eg * sm.rk[tid];
+    }
+    __syncthreads();
+    if (tid < kC) sm.ed[tid] = expf(sm.G[kC - 1] - sm.G[tid]);
     {
-      // forward substitution, one column of [beta v | beta exp(G) k^] per thread
-      const int c = tid & 127;
-      const bool vhalf = tid < 128;
-      float x[kC];
-      if (vhalf) {
-        const __nv_bfloat16* vp = mixed_b + 2 * gm.Hqk * kD + hv * kD + c;
+      const float G_lo = sm.G[row_lo], G_hi = sm.G[row_hi], b_lo = sm.beta[row_lo], b_hi = sm.beta[row_hi];
+      __nv_bfloat16* intra = p.intra + chunk * kC * kC;
 #pragma unroll
-        for (int i = 0; i < kC; ++i) {
-          const int t = n * kC + i;
-          x[i] = t < gm.T ? s_beta[i] * bf2f(vp + static_cast<size_t>(t) * gm.conv_dim) : 0.f;
+      for (int j = 0; j < 8; ++j) {
+        const int c0 = j * 8 + 2 * t4, c1 = c0 + 1;
+        const float2 Gc = *reinterpret_cast<const float2*>(sm.G + c0);
+        if (of_q) {
+          const float w00 = c0 <= row_lo ? gram[j][0] * expf(G_lo - Gc.x) : 0.f, w01 = c1 <= row_lo ? gram[j][1] * expf(G_lo - Gc.y) : 0.f;
+          const float w10 = c0 <= row_hi ? gram[j][2] * expf(G_hi - Gc.x) : 0.f, w11 = c1 <= row_hi ? gram[j][3] * expf(G_hi - Gc.y) : 0.f;
+          *reinterpret_cast<uint32_t*>(intra + row_lo * kC + c0) = pack_bf16x2(w00, w01);
+          *reinterpret_cast<uint32_t*>(intra + row_hi * kC + c0) = pack_bf16x2(w10, w11);
+        } else {
+          const float a00 = c0 < row_lo ? b_lo * gram[j][0] * expf(G_lo - Gc.x) : 0.f, a01 = c1 < row_lo ? b_lo * gram[j][1] * expf(G_lo - Gc.y) : 0.f;
+          const float a10 = c0 < row_hi ? b_hi * gram[j][2] * expf(G_hi - Gc.x) : 0.f, a11 = c1 < row_hi ? b_hi * gram[j][3] * expf(G_hi - Gc.y) : 0.f;
+          *reinterpret_cast<float2*>(sm.A + row_lo * kALd + c0) = make_float2(a00, a01);
+          *reinterpret_cast<float2*>(sm.A + row_hi * kALd + c0) = make_float2(a10, a11);
         }
-      } else {
-#pragma unroll
-        for (int i = 0; i < kC; ++i) x[i] = s_beta[i] * s_eg[i] * sk[i * kLd + c];
       }
+    }
+    __syncthreads();
+    unit_lower_inverse(sm.A, sm.T, sm.U);
+    {
+      // X = (T diag(s)) R: warps 0-3 the value columns (s = beta), warps 4-7 the key columns (s = beta exp(G) / |k|), 32 columns each
+      const __nv_bfloat16* right = (of_q ? sm.k : sm.v) + mt * 32;
+      const float* scale = of_q ? sm.kscale : sm.beta;
+      __nv_bfloat16* out = (of_q ? p.kq + chunk * 2 * kC * kD : p.veff + chunk * kC * kD) + mt * 32;
 #pragma unroll
-      for (int i = 1; i < kC; ++i) {
-        float acc = 0.f;
+      for (int m = 0; m < 4; ++m) {
+        float acc[4][4];
 #pragma unroll
-        for (int j4 = 0; j4 * 4 < i; ++j4) {
-          const float4 m = *reinterpret_cast<const float4*>(sA + i * kC + 4 * j4);   // entries at or right of the diagonal are 0
-          acc += m.x * x[4 * j4] + m.y * x[4 * j4 + 1] + m.z * x[4 * j4 + 2] + m.w * x[4 * j4 + 3];
+        for (int j = 0; j < 4; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks) {
+          if (ks > m) continue;
+          uint32_t part[3][4];
+#pragma unroll
+          for (int f = 0; f < 4; ++f) {     // fragment registers: rows g, g + 8, columns 2 t4 and 8 further
+            const int row = m * 16 + g + (f & 1) * 8, col = ks * 16 + 2 * t4 + (f >> 1) * 8;
+            float2 x = *reinterpret_cast<const float2*>(sm.T + row * kTLd + col);
+            const float2 s = *reinterpret_cast<const float2*>(scale + col);
+            x.x *= s.x;
+            x.y *= s.y;
+#pragma unroll
+            for (int e = 0; e < 3; ++e) {
+              part[e][f] = pack_bf16x2(x.x, x.y);
+              const float2 h = unpack_bf16x2(part[e][f]);
+              x.x -= h.x;
+              x.y -= h.y;
+            }
+          }
+#pragma unroll
+          for (int j2 = 0; j2 < 2; ++j2) {
+            uint32_t b[4];
+            ldsm4_t(b, right + (ks * 16 + ((lane >> 3) & 1) * 8 + (lane & 7)) * kRawLd + j2 * 16 + (lane >> 4) * 8);
+#pragma unroll
+            for (int e = 2; e >= 0; --e) {  // the small parts first
+              mma_16816(acc[2 * j2], part[e], b[0], b[1]);
+              mma_16816(acc[2 * j2 + 1], part[e], b[2], b[3]);
+            }
+          }
         }
-        x[i] -= acc;
-      }
-      __nv_bfloat16* out = vhalf ? p.veff + chunk * kC * kD + c : p.kq + chunk * 2 * kC * kD + c;
 #pragma unroll
-      for (int i = 0; i < kC; ++i) out[i * kD] = __float2bfloat16(x[i]);
+        for (int j = 0; j < 4; ++j) {
+          *reinterpret_cast<uint32_t*>(out + (m * 16 + g) * kD + j * 8 + 2 * t4) = pack_bf16x2(acc[j][0], acc[j][1]);
+          *reinterpret_cast<uint32_t*>(out + (m * 16 + g + 8) * kD + j * 8 + 2 * t4) = pack_bf16x2(acc[j][2], acc[j][3]);
+        }
+      }
     }
-    for (int idx = tid; idx < kC * (kD / 2); idx += kThreads) {
-      const int i = idx >> 6, c2 = idx & 63;
-      const float2 q2 = *reinterpret_cast<const float2*>(sq + i * kLd + 2 * c2);
-      const float2 k2 = *reinterpret_cast<const float2*>(sk + i * kLd + 2 * c2);
-      const float eg = s_eg[i], ed = s_ed[i];
-      *reinterpret_cast<__nv_bfloat162*>(p.kq + (chunk * 2 * kC + kC + i) * kD + 2 * c2) =
-          __floats2bfloat162_rn(q2.x * eg, q2.y * eg);
-      *reinterpret_cast<__nv_bfloat162*>(p.kdec + (chunk * kC + i) * kD + 2 * c2) =
-          __floats2bfloat162_rn(k2.x * ed, k2.y * ed);
+    for (int idx = tid; idx < kC * (kD / 8); idx += kThreads) {
+      const int i = idx >> 4, c8 = idx & 15;
+      const uint4 q8 = *reinterpret_cast<const uint4*>(sm.q + i * kRawLd + c8 * 8);
+      const uint4 k8 = *reinterpret_cast<const uint4*>(sm.k + i * kRawLd + c8 * 8);
+      const float rq = sm.rq[i], rk = sm.rk[i], eg = sm.eg[i], ed = sm.ed[i];
+      const uint32_t qw[4] = {q8.x, q8.y, q8.z, q8.w}, kw[4] = {k8.x, k8.y, k8.z, k8.w};
+      uint32_t qo[4], ko[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 x = unpack_bf16x2(qw[e]), y = unpack_bf16x2(kw[e]);
+        qo[e] = pack_bf16x2(x.x * rq * eg, x.y * rq * eg);
+        ko[e] = pack_bf16x2(y.x * rk * ed, y.y * rk * ed);
+      }
+      *reinterpret_cast<uint4*>(p.kq + (chunk * 2 * kC + kC + i) * kD + c8 * 8) = make_uint4(qo[0], qo[1], qo[2], qo[3]);
+      *reinterpret_cast<uint4*>(p.kdec + (chunk * kC + i) * kD + c8 * 8) = make_uint4(ko[0], ko[1], ko[2], ko[3]);
     }
-    if (tid == 0) p.e[chunk] = s_eg[kC - 1];
+    if (tid == 0) p.e[chunk] = sm.eg[kC - 1];
     __syncthreads();
   }
 }
@@ -703,7 +913,7 @@ cudaError_t launch_gdn_chunk_prep(const __nv_bfloat16* mixed, const __nv_bfloat1
                                   cudaStream_t stream) {
   if (!prep_geom_ok(B, T, Hqk, Hv)) return cudaErrorInvalidValue;
   const int N = (T + kC - 1) / kC;
-  constexpr int smem = kFwdSmemFloats * 4;
+  constexpr int smem = sizeof(PrepFwdSmem);
   static bool configured = false;
   if (!configured) {
     cudaError_t err = cudaFuncSetAttribute(gdn_chunk_prep_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);

@@ -431,6 +431,12 @@ def test_gdn_chunk_prep_kernel(cuda_device, B, T, n_qk, n_v):
         assert _rel(got.float().cpu(), ref) < 8e-3, (name, _rel(got.float().cpu(), ref))
 
 
+@pytest.mark.parametrize("B,T,n_qk,n_v", [(1, 1, 2, 4), (3, 63, 1, 8), (1, 65, 2, 2), (1, 127, 1, 3)])
+def test_gdn_chunk_prep_kernel_edges(cuda_device, B, T, n_qk, n_v):
+    """One token, a chunk that is one short, one token and all but one of a second chunk, several value heads per qk head."""
+    test_gdn_chunk_prep_kernel(cuda_device, B, T, n_qk, n_v)
+
+
 @pytest.mark.parametrize("B,T,n_qk,n_v,with_state", [(1, 128, 1, 1, False), (2, 200, 2, 4, True)])
 def test_gated_delta_prefill_cuda_gradients(cuda_device, B, T, n_qk, n_v, with_state):
     """The whole prefill on the kernels (chunk preparation + inter-chunk scan, forward and backward) against
