@@ -9,14 +9,18 @@
 //     o     = (q * exp(G)) S + intra v_new
 //     S     = exp(g_end) S + (k * exp(g_end - G))^T v_new
 // which the reference runs as a `lax.scan` over chunks (jax_gpt/models/qwen35/deltanet.py:300-360).
-// Here one CTA per (batch, head) walks the chunks with S resident on chip: fp32 in the registers of
-// 128 threads (one row of the 128 x 128 state each), a bf16 copy in shared memory as tensor-core
-// operand. Per chunk three MMAs:
-//   1. D[128 x 128] = [k_cum ; q exp(G)] S      (the two 64-row operands stacked to M = 128)
-//   2. D[64:128]   += [0 ; intra] v_new         (A tile with a zero upper half)
-//   3. P[128 x 128] = (k exp(g_end - G))^T v_new
-// with v_new produced between 1 and 2 by the threads that own rows 0..63 of D. TMA double-buffers
-// the per-chunk operand tiles.
+// Here two CTAs per (batch, head) walk the chunks, each with half of the value columns (the columns of S do
+// not depend on one another), S resident on chip: fp32 in the registers of 256 threads (half a row of the
+// 128 x 64 part each), a bf16 copy in shared memory as tensor-core operand. Per chunk three MMAs:
+//   1. D[128 x 64] = [k_cum ; q exp(G)] S      (the two 64-row operands stacked to M = 128)
+//   2. P[128 x 64] = (k exp(g_end - G))^T v_new
+//   3. D[64:128]  += [0 ; intra] v_new         (A tile with a zero upper half)
+// with v_new produced after 1 by the threads that own rows 0..63 of D.
+//
+// What bounds it is the chain of a chunk: product 1, v_new, product 2, the new S. One CTA per head with a row
+// of 128 columns per thread took 3.5 us a chunk (4096 tokens, 32 heads: 228 us); the halves are 32 columns a
+// thread, the outputs leave the chain (D is double-buffered, they are read while the next chunk runs), the
+// corrected values are fetched a chunk ahead and three stages of operand tiles cover the loads: 102 us.
 #include "seq_kernels.cuh"
 
 #include "common.cuh"
@@ -27,18 +31,20 @@ namespace b200 {
 namespace {
 
 constexpr int kC = 64, kDk = 128, kDv = 128;
-constexpr int kStages = 2;
+constexpr int kStages = 3;
+constexpr int kCols = 64;                       // value columns of a CTA
 constexpr int kA1Bytes = 128 * kDk * 2;      // 32 KB  [k_cum ; qg], two 64-column K blocks of 16 KB
 constexpr int kA2Bytes = 128 * kC * 2;       // 16 KB  [0 ; intra]
 constexpr int kKdBytes = kC * kDk * 2;       // 16 KB  k_dec, two 64-column blocks of 8 KB
 constexpr int kStageBytes = kA1Bytes + kA2Bytes + kKdBytes;   // 64 KB
-constexpr int kSbBytes = kDk * kDv * 2;      // 32 KB  S as bf16, two 64-column blocks of 16 KB
-constexpr int kVnBytes = kC * kDv * 2;       // 16 KB  v_new, two 64-column blocks of 8 KB
-constexpr int kThreads = 192;
+constexpr int kSbBytes = kDk * kCols * 2;    // 16 KB  S as bf16
+constexpr int kVnBytes = kC * kCols * 2;     // 8 KB   v_new
+constexpr int kRowThreads = 256;             // two per row of D / P / S, 32 columns each
+constexpr int kThreads = 64 + kRowThreads;
 constexpr int kSmem = 1024 + kStages * kStageBytes + kSbBytes + kVnBytes + 256;
 
 struct ScanBars {
-  uint64_t full[kStages], empty[kStages], d_full, vn_ready, p_full, s_ready;
+  uint64_t full[kStages], empty[kStages], d_full, vn_ready, p_full, o_full, s_ready;
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -70,7 +76,7 @@ gdn_scan_kernel(const __grid_constant__ CUtensorMap t_kq, const __grid_constant_
   ScanBars* bars = reinterpret_cast<ScanBars*>(vn + kVnBytes);
   volatile int* abort_flag = &bars->abort_flag;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int bh = blockIdx.x;
+  const int bh = blockIdx.x, col0 = blockIdx.y * kCols;
   const int N = a.n_chunks;
 
   if (threadIdx.x == 0) {
@@ -79,9 +85,10 @@ gdn_scan_kernel(const __grid_constant__ CUtensorMap t_kq, const __grid_constant_
       mbar_init(&bars->empty[s], 1);
     }
     mbar_init(&bars->d_full, 1);
-    mbar_init(&bars->vn_ready, 128);
+    mbar_init(&bars->vn_ready, kRowThreads);
     mbar_init(&bars->p_full, 1);
-    mbar_init(&bars->s_ready, 128);
+    mbar_init(&bars->o_full, 1);
+    mbar_init(&bars->s_ready, kRowThreads);
     bars->abort_flag = 0;
     fence_mbar_init();
   }
@@ -98,15 +105,16 @@ gdn_scan_kernel(const __grid_constant__ CUtensorMap t_kq, const __grid_constant_
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = bars->tmem_base;
+  const uint32_t tmem = bars->tmem_base;      // D of even and odd chunks, then P: 64 columns each
+  constexpr uint32_t kColP = 2 * kCols;
 
   if (warp == 0) {
     if (elect_one()) {
       bool ok = true;
       int issued = 0;
       for (int n = 0; n < N; ++n, ++issued) {
-        const int st = n & 1;
-        if (n >= kStages && !mbar_wait(&bars->empty[st], ((n >> 1) - 1) & 1, abort_flag)) {
+        const int st = n % kStages;
+        if (n >= kStages && !mbar_wait(&bars->empty[st], (n / kStages - 1) & 1, abort_flag)) {
           report_status(a.status, kWaitEmptyTimeout, 100, bh, n);
           ok = false;
           break;
@@ -124,7 +132,7 @@ gdn_scan_kernel(const __grid_constant__ CUtensorMap t_kq, const __grid_constant_
         // leave no bulk copy in flight: wait (bounded) for the last fill of each stage to land
         const uint64_t tw = globaltimer_ns();
         for (int s = 0; s < kStages; ++s) {
-          const int uses = (issued + 1 - s) / 2;
+          const int uses = (issued + kStages - 1 - s) / kStages;
           if (uses > 0)
             while (!mbar_try_wait(&bars->full[s], (uses - 1) & 1) && globaltimer_ns() - tw < 2000000ull) {
             }
@@ -133,20 +141,21 @@ gdn_scan_kernel(const __grid_constant__ CUtensorMap t_kq, const __grid_constant_
     }
   } else if (warp == 1) {
     if (elect_one()) {   // one thread waits and issues
-      constexpr uint32_t idesc_kn = make_idesc(128, 128, 0, 1, 1);   // A K-major, B MN-major
-      constexpr uint32_t idesc_nn = make_idesc(128, 128, 1, 1, 1);   // both MN-major
+      constexpr uint32_t idesc_kn = make_idesc(128, kCols, 0, 1, 1);   // A K-major, B MN-major
+      constexpr uint32_t idesc_nn = make_idesc(128, kCols, 1, 1, 1);   // both MN-major
       const uint32_t a_sb = smem_u32(sb), a_vn = smem_u32(vn);
       for (int n = 0; n < N; ++n) {
-        const int st = n & 1;
+        const int st = n % kStages;
         const uint32_t a1 = smem_u32(smem + st * kStageBytes), a2 = a1 + kA1Bytes, kd = a2 + kA2Bytes;
-        if (!mbar_wait(&bars->s_ready, n & 1, abort_flag) || !mbar_wait(&bars->full[st], (n >> 1) & 1, abort_flag)) {
+        const uint32_t d = tmem + (n & 1) * kCols;
+        if (!mbar_wait(&bars->s_ready, n & 1, abort_flag) || !mbar_wait(&bars->full[st], (n / kStages) & 1, abort_flag)) {
           report_status(a.status, kWaitFullTimeout, 101, bh, n);
           break;
         }
         tc_fence_after();
 #pragma unroll
         for (int k = 0; k < 8; ++k)   // K = dk = 128: block k / 4, 32 bytes per step
-          umma_bf16(tmem, make_smem_desc(a1 + (k >> 2) * 16384 + (k & 3) * 32, 16, 1024),
+          umma_bf16(d, make_smem_desc(a1 + (k >> 2) * 16384 + (k & 3) * 32, 16, 1024),
                     make_smem_desc(a_sb + k * 2048, 16384, 1024), idesc_kn, k > 0 ? 1u : 0u);
         tc_commit(&bars->d_full);
         if (!mbar_wait(&bars->vn_ready, n & 1, abort_flag)) {
@@ -155,126 +164,135 @@ gdn_scan_kernel(const __grid_constant__ CUtensorMap t_kq, const __grid_constant_
         }
         tc_fence_after();
 #pragma unroll
-        for (int k = 0; k < 4; ++k)   // K = 64 tokens
-          umma_bf16(tmem, make_smem_desc(a2 + k * 32, 16, 1024), make_smem_desc(a_vn + k * 2048, 8192, 1024), idesc_kn, 1u);
+        for (int k = 0; k < 4; ++k)   // K = 64 tokens; the state first, the next chunk waits for it
+          umma_bf16(tmem + kColP, make_smem_desc(kd + k * 2048, 8192, 1024), make_smem_desc(a_vn + k * 2048, 8192, 1024),
+                    idesc_nn, k > 0 ? 1u : 0u);
+        tc_commit(&bars->p_full);
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-          umma_bf16(tmem + 128, make_smem_desc(kd + k * 2048, 8192, 1024), make_smem_desc(a_vn + k * 2048, 8192, 1024),
-                    idesc_nn, k > 0 ? 1u : 0u);
+          umma_bf16(d, make_smem_desc(a2 + k * 32, 16, 1024), make_smem_desc(a_vn + k * 2048, 8192, 1024), idesc_kn, 1u);
         tc_commit(&bars->empty[st]);
-        tc_commit(&bars->p_full);
+        tc_commit(&bars->o_full);
       }
     }
   } else {
-    const int q = warp & 3;
-    const int r = q * 32 + lane;                     // row of D / P / S owned by this thread
+    const int q = warp & 3, c0 = ((warp - 2) >> 2) * 32;   // TMEM lane quarter, first of this thread's columns of the CTA's part
+    const int r = q * 32 + lane;                           // row of D / P / S
     const uint32_t lane_off = static_cast<uint32_t>(q * 32) << 16;
-    float S[kDv];
+    const bool token = r < kC;                             // rows 0..63 of D: v_new of a token, rows 64..127: its output
+    float S[32];
     if (a.s0 != nullptr) {
-      const float4* sp = reinterpret_cast<const float4*>(a.s0 + (static_cast<int64_t>(bh) * kDk + r) * kDv);
+      const float4* sp = reinterpret_cast<const float4*>(a.s0 + (static_cast<int64_t>(bh) * kDk + r) * kDv + col0 + c0);
 #pragma unroll
-      for (int j = 0; j < kDv / 4; ++j) {
+      for (int j = 0; j < 8; ++j) {
         const float4 f = sp[j];
         S[4 * j] = f.x; S[4 * j + 1] = f.y; S[4 * j + 2] = f.z; S[4 * j + 3] = f.w;
       }
     } else {
 #pragma unroll
-      for (int j = 0; j < kDv; ++j) S[j] = 0.f;
+      for (int j = 0; j < 32; ++j) S[j] = 0.f;
     }
-    bool ok = true;
-    for (int n = 0; n <= N; ++n) {
-      // ---- publish S (bf16) for the next chunk's first product ----
-      if (n < N) {
-        uint4* ssave = a.s_save != nullptr
-                           ? reinterpret_cast<uint4*>(a.s_save + ((static_cast<int64_t>(bh) * N + n) * kDk + r) * kDv)
-                           : nullptr;
+    auto publish = [&](int n) {       // S as bf16: the operand of chunk n
+      uint4* ssave = a.s_save != nullptr ? reinterpret_cast<uint4*>(a.s_save + ((static_cast<int64_t>(bh) * N + n) * kDk + r) * kDv + col0 + c0)
+                                         : nullptr;
 #pragma unroll
-        for (int c = 0; c < kDv; c += 8) {
-          const uint4 pk = make_uint4(pack_bf16x2(S[c], S[c + 1]), pack_bf16x2(S[c + 2], S[c + 3]),
-                                      pack_bf16x2(S[c + 4], S[c + 5]), pack_bf16x2(S[c + 6], S[c + 7]));
-          *reinterpret_cast<uint4*>(sb + swz(r, c, 16384)) = pk;
-          if (ssave != nullptr) ssave[c >> 3] = pk;
-        }
-        fence_proxy_async_smem();
-        mbar_arrive(&bars->s_ready);
-      } else {
-        break;
+      for (int c = 0; c < 32; c += 8) {
+        const uint4 pk = make_uint4(pack_bf16x2(S[c], S[c + 1]), pack_bf16x2(S[c + 2], S[c + 3]),
+                                    pack_bf16x2(S[c + 4], S[c + 5]), pack_bf16x2(S[c + 6], S[c + 7]));
+        *reinterpret_cast<uint4*>(sb + swz(r, c0 + c, 16384)) = pk;
+        if (ssave != nullptr) ssave[c >> 3] = pk;
       }
+      fence_proxy_async_smem();
+      mbar_arrive(&bars->s_ready);
+    };
+    uint4 ve[4];                      // this token's corrected values, fetched a chunk ahead
+    float e = 0.f;
+    auto fetch = [&](int n) {
       const int64_t chunk = static_cast<int64_t>(bh) * N + n;
-      // rows 0..63 own a token of the chunk: fetch its corrected value early
-      uint4 ve[16];
-      if (r < kC) {
-        const uint4* vp = reinterpret_cast<const uint4*>(a.veff + (chunk * kC + r) * kDv);
+      if (token) {
+        const uint4* vp = reinterpret_cast<const uint4*>(a.veff + (chunk * kC + r) * kDv + col0 + c0);
 #pragma unroll
-        for (int j = 0; j < 16; ++j) ve[j] = __ldg(vp + j);
+        for (int j = 0; j < 4; ++j) ve[j] = __ldg(vp + j);
       }
-      const float e = a.e[chunk];
-      if (ok && !mbar_wait(&bars->d_full, n & 1, abort_flag)) {
-        if (lane == 0) report_status(a.status, kWaitTmemFullTimeout, 103, bh, n);
-        ok = false;
-      }
-      ok = __all_sync(0xffffffffu, ok);
-      if (ok && r < kC) {
-        tc_fence_after();
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
+      e = a.e[chunk];
+    };
+    publish(0);
+    fetch(0);
+    bool ok = true;
+    for (int n = 0; n < N; ++n) {
+      const int64_t chunk = static_cast<int64_t>(bh) * N + n;
+      const uint32_t d = tmem + (n & 1) * kCols + c0 + lane_off;
+      if (token) {                    // whole warps: a quarter's rows are on one side
+        if (ok && !mbar_wait(&bars->d_full, n & 1, abort_flag)) {
+          if (lane == 0) report_status(a.status, kWaitTmemFullTimeout, 103, bh, n);
+          ok = false;
+        }
+        ok = __all_sync(0xffffffffu, ok);
+        if (ok) {
+          tc_fence_after();
           uint32_t v[32];
-          tmem_ld_32x32(tmem + c * 32 + lane_off, v);
+          tmem_ld_32x32(d, v);
           tmem_ld_wait();
 #pragma unroll
           for (int j = 0; j < 32; j += 8) {
-            const uint4 u = ve[c * 4 + (j >> 3)];
+            const uint4 u = ve[j >> 3];
             const float2 f0 = unpack_bf16x2(u.x), f1 = unpack_bf16x2(u.y), f2 = unpack_bf16x2(u.z), f3 = unpack_bf16x2(u.w);
             const uint4 pk = make_uint4(
                 pack_bf16x2(f0.x - __uint_as_float(v[j]), f0.y - __uint_as_float(v[j + 1])),
                 pack_bf16x2(f1.x - __uint_as_float(v[j + 2]), f1.y - __uint_as_float(v[j + 3])),
                 pack_bf16x2(f2.x - __uint_as_float(v[j + 4]), f2.y - __uint_as_float(v[j + 5])),
                 pack_bf16x2(f3.x - __uint_as_float(v[j + 6]), f3.y - __uint_as_float(v[j + 7])));
-            *reinterpret_cast<uint4*>(vn + swz(r, c * 32 + j, 8192)) = pk;
-            if (a.vn_save != nullptr)
-              reinterpret_cast<uint4*>(a.vn_save + (chunk * kC + r) * kDv)[c * 4 + (j >> 3)] = pk;
+            *reinterpret_cast<uint4*>(vn + swz(r, c0 + j, 8192)) = pk;
+            if (a.vn_save != nullptr) reinterpret_cast<uint4*>(a.vn_save + (chunk * kC + r) * kDv + col0 + c0)[j >> 3] = pk;
           }
+          tc_fence_before();
+          fence_proxy_async_smem();
         }
-        tc_fence_before();
-        fence_proxy_async_smem();
       }
       mbar_arrive(&bars->vn_ready);
+      const float e_now = e;
+      if (n + 1 < N) fetch(n + 1);
       if (ok && !mbar_wait(&bars->p_full, n & 1, abort_flag)) {
         if (lane == 0) report_status(a.status, kWaitTmemFullTimeout, 104, bh, n);
         ok = false;
       }
       ok = __all_sync(0xffffffffu, ok);
-      if (!ok) continue;
-      tc_fence_after();
-      if (r >= kC) {   // rows 64..127 of D are the chunk's outputs
-        uint4* op = reinterpret_cast<uint4*>(a.o + (chunk * kC + (r - kC)) * kDv);
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          uint32_t v[32];
-          tmem_ld_32x32(tmem + c * 32 + lane_off, v);
-          tmem_ld_wait();
-#pragma unroll
-          for (int j = 0; j < 32; j += 8)
-            op[c * 4 + (j >> 3)] = make_uint4(pack_bf16x2(__uint_as_float(v[j]), __uint_as_float(v[j + 1])),
-                                               pack_bf16x2(__uint_as_float(v[j + 2]), __uint_as_float(v[j + 3])),
-                                               pack_bf16x2(__uint_as_float(v[j + 4]), __uint_as_float(v[j + 5])),
-                                               pack_bf16x2(__uint_as_float(v[j + 6]), __uint_as_float(v[j + 7])));
-        }
-      }
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
+      if (ok) {
+        tc_fence_after();
         uint32_t v[32];
-        tmem_ld_32x32(tmem + 128 + c * 32 + lane_off, v);
+        tmem_ld_32x32(tmem + kColP + c0 + lane_off, v);
         tmem_ld_wait();
 #pragma unroll
-        for (int j = 0; j < 32; ++j) S[c * 32 + j] = S[c * 32 + j] * e + __uint_as_float(v[j]);
+        for (int j = 0; j < 32; ++j) S[j] = S[j] * e_now + __uint_as_float(v[j]);
+        tc_fence_before();
       }
-      tc_fence_before();
+      if (n + 1 < N) publish(n + 1);
+      if (!token) {                   // the outputs: D of this chunk is not written before the chunk after the next
+        if (ok && !mbar_wait(&bars->o_full, n & 1, abort_flag)) {
+          if (lane == 0) report_status(a.status, kWaitTmemFullTimeout, 105, bh, n);
+          ok = false;
+        }
+        ok = __all_sync(0xffffffffu, ok);
+        if (ok) {
+          tc_fence_after();
+          uint32_t v[32];
+          tmem_ld_32x32(d, v);
+          tmem_ld_wait();
+          uint4* op = reinterpret_cast<uint4*>(a.o + (chunk * kC + (r - kC)) * kDv + col0 + c0);
+#pragma unroll
+          for (int j = 0; j < 32; j += 8)
+            op[j >> 3] = make_uint4(pack_bf16x2(__uint_as_float(v[j]), __uint_as_float(v[j + 1])),
+                                    pack_bf16x2(__uint_as_float(v[j + 2]), __uint_as_float(v[j + 3])),
+                                    pack_bf16x2(__uint_as_float(v[j + 4]), __uint_as_float(v[j + 5])),
+                                    pack_bf16x2(__uint_as_float(v[j + 6]), __uint_as_float(v[j + 7])));
+          tc_fence_before();
+        }
+      }
     }
     if (ok) {
-      float4* sp = reinterpret_cast<float4*>(a.s_out + (static_cast<int64_t>(bh) * kDk + r) * kDv);
+      float4* sp = reinterpret_cast<float4*>(a.s_out + (static_cast<int64_t>(bh) * kDk + r) * kDv + col0 + c0);
 #pragma unroll
-      for (int j = 0; j < kDv / 4; ++j) sp[j] = make_float4(S[4 * j], S[4 * j + 1], S[4 * j + 2], S[4 * j + 3]);
+      for (int j = 0; j < 8; ++j) sp[j] = make_float4(S[4 * j], S[4 * j + 1], S[4 * j + 2], S[4 * j + 3]);
     }
   }
   tc_fence_before();
@@ -553,7 +571,7 @@ cudaError_t launch_gdn_scan(const __nv_bfloat16* kq, const __nv_bfloat16* intra,
     configured = true;
   }
   ScanArgs args{n_chunks, veff, e, s0, o, s_out, s_save, vn_save, status};
-  gdn_scan_kernel<<<bh, kThreads, kSmem, stream>>>(t_kq, t_intra, t_kdec, args);
+  gdn_scan_kernel<<<dim3(bh, kDv / kCols), kThreads, kSmem, stream>>>(t_kq, t_intra, t_kdec, args);
   return cudaGetLastError();
 }
 
