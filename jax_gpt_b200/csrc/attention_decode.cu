@@ -48,6 +48,31 @@ struct DecArgs {
   SoftCap cap;              // kCap instances
 };
 
+// Merges a CTA's warps and writes the partial result of its key range.
+template <int DV, int G>
+__device__ __forceinline__ void merge_warps(const DecArgs& a, const float (&sm_o)[kDecWarps][G][DV], const float (&sm_m)[kDecWarps][G],
+                                            const float (&sm_l)[kDecWarps][G], int b, int hkv, int split, int n_splits) {
+  for (int i = threadIdx.x; i < G * DV; i += kDecWarps * 32) {
+    const int g = i / DV, c = i % DV;
+    float mn = -INFINITY;
+#pragma unroll
+    for (int w = 0; w < kDecWarps; ++w) mn = fmaxf(mn, sm_m[w][g]);
+    float acc = 0.f, ls = 0.f;
+#pragma unroll
+    for (int w = 0; w < kDecWarps; ++w) {
+      const float wt = (sm_m[w][g] == -INFINITY) ? 0.f : exp2f(sm_m[w][g] - mn);
+      acc = fmaf(sm_o[w][g][c], wt, acc);
+      ls = fmaf(sm_l[w][g], wt, ls);
+    }
+    const int64_t row = (static_cast<int64_t>(b) * a.H + hkv * G + g) * n_splits + split;
+    a.part_o[row * DV + c] = acc;
+    if (c == 0) {
+      a.part_ml[row * 2] = mn;
+      a.part_ml[row * 2 + 1] = ls;
+    }
+  }
+}
+
 // D: query and key width, DV: value width (D or 2 D).
 template <int D, int DV, int G, bool kCap, bool kPool>
 __global__ void __launch_bounds__(kDecWarps * 32)
@@ -198,25 +223,160 @@ attn_decode_split_kernel(const DecArgs a) {
     }
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < G * DV; i += kDecWarps * 32) {
-    const int g = i / DV, c = i % DV;
-    float mn = -INFINITY;
+  merge_warps<DV, G>(a, sm_o, sm_m, sm_l, b, hkv, split, n_splits);
+}
+
+// The same for four or eight query heads per kv head, on matrix instructions. The kernel above shares a key row among 8 - 32 lanes and
+// sums every score over them: with eight queries of 256 that is 40 shuffles and 300 instructions a key, which bounded it at a sixth
+// of the copy rate. Here a warp takes 16 keys a step; both products have the keys' or values' rows as the 16-row operand and the
+// (up to eight) queries as the columns, and the fragments come straight from global memory:
+//   scores [16 keys x 8]     the order of the features inside a product is free, so a lane's 16 bytes of a row are its columns of two steps;
+//   output [features x 8]    the transposed values: a lane holds 8 features of 4 keys, packed pairwise by key.
+// The probabilities stay fp32-exact to 2^-17: high and low bf16 part, two products. Key rows past the range are zeros.
+// 32 sequences x 2048 keys, 2 kv heads of 256, 8 queries each (134 MB, 21 us): 141 -> 42 us;
+// 8 sequences x 700 keys, 2 kv heads of 128: 12 -> 6.3 us.
+__device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint32_t transpose_8x8(uint32_t v) {   // of a bf16 matrix whose row g, columns 2 t and 2 t + 1 lane 4 g + t holds
+  uint32_t r;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(v));
+  return r;
+}
+
+template <int D, int DV, int G, bool kCap>
+__global__ void __launch_bounds__(kDecWarps * 32)
+attn_decode_mma_kernel(const DecArgs a) {
+  constexpr int kStep = 16, KS = D / 32, VS = DV / 64;
+  __shared__ float sm_o[kDecWarps][G][DV];
+  __shared__ float sm_m[kDecWarps][G], sm_l[kDecWarps][G];
+  const int split = blockIdx.x, hkv = blockIdx.y, b = blockIdx.z;
+  const int n_splits = gridDim.x;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int seq = a.table != nullptr ? a.seq_ids[b] : b;
+  const int len = a.table != nullptr ? a.lens[seq] + a.len_add : (a.pos_ptr != nullptr ? a.pos_ptr[0] + a.len_add : a.len);
+  const int* pages = a.table != nullptr ? a.table + static_cast<int64_t>(seq) * a.max_pages : nullptr;
+  // the seen keys numbered through: the kept first ones, then the window (see the kernel above)
+  const int n_keep = a.window > 0 ? min(a.keep_first, len) : 0;
+  const int w0 = a.window > 0 ? max(n_keep, len - a.window) : 0;
+  const int n_seen = n_keep + len - w0;
+  const int per = ((n_seen + n_splits - 1) / n_splits + kStep * kDecWarps - 1) / (kStep * kDecWarps) * (kStep * kDecWarps);
+  const int k0 = split * per, k1 = min(n_seen, k0 + per);
+
+  uint32_t qf[KS][4];   // query g (zero past G): its columns of two steps per 32 features
 #pragma unroll
-    for (int w = 0; w < kDecWarps; ++w) mn = fmaxf(mn, sm_m[w][g]);
-    float acc = 0.f, ls = 0.f;
+  for (int s = 0; s < KS; ++s) {
+    uint4 u = make_uint4(0, 0, 0, 0);
+    if (g < G) u = *reinterpret_cast<const uint4*>(a.q + static_cast<int64_t>(b) * a.ldq + (hkv * G + g) * D + 32 * s + 8 * t);
+    qf[s][0] = u.x;
+    qf[s][1] = u.y;
+    qf[s][2] = u.z;
+    qf[s][3] = u.w;
+  }
+  float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;   // of queries 2 t and 2 t + 1
+  float o[VS][4][4];
 #pragma unroll
-    for (int w = 0; w < kDecWarps; ++w) {
-      const float wt = (sm_m[w][g] == -INFINITY) ? 0.f : exp2f(sm_m[w][g] - mn);
-      acc = fmaf(sm_o[w][g][c], wt, acc);
-      ls = fmaf(sm_l[w][g], wt, ls);
+  for (int u = 0; u < VS; ++u)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) o[u][j][0] = o[u][j][1] = o[u][j][2] = o[u][j][3] = 0.f;
+  const __nv_bfloat16* kb = a.k + (pages == nullptr ? b * a.kv_stride_b : 0) + hkv * a.kv_stride_h + 8 * t;
+  const __nv_bfloat16* vb = a.v + (pages == nullptr ? b * a.kv_stride_b : 0) + hkv * a.v_stride_h + 8 * g;
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  for (int base = k0 + warp * kStep; base < k1; base += kStep * kDecWarps) {
+    int row = 0;   // cache row of key base + lane % 16
+    {
+      int key = base + (lane & 15);
+      if (key < k1) {
+        if (key >= n_keep) key += w0 - n_keep;
+        row = pages == nullptr ? key : pages[key / a.page_size] * a.page_size + key % a.page_size;
+      }
     }
-    const int64_t row = (static_cast<int64_t>(b) * a.H + hkv * G + g) * n_splits + split;
-    a.part_o[row * DV + c] = acc;
-    if (c == 0) {
-      a.part_ml[row * 2] = mn;
-      a.part_ml[row * 2 + 1] = ls;
+    uint4 ku[2][KS], vu[4][VS];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const bool has = base + g + 8 * h < k1;
+      const __nv_bfloat16* p = kb + static_cast<int64_t>(__shfl_sync(0xffffffffu, row, g + 8 * h)) * a.kv_stride_t;
+#pragma unroll
+      for (int s = 0; s < KS; ++s) ku[h][s] = has ? *reinterpret_cast<const uint4*>(p + 32 * s) : zero;
+    }
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      const int key = 2 * t + (h & 1) + 8 * (h >> 1);
+      const bool has = base + key < k1;
+      const __nv_bfloat16* p = vb + static_cast<int64_t>(__shfl_sync(0xffffffffu, row, key)) * a.kv_stride_t;
+#pragma unroll
+      for (int u = 0; u < VS; ++u) vu[h][u] = has ? *reinterpret_cast<const uint4*>(p + 64 * u) : zero;
+    }
+    float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int i = 0; i < KS; ++i) {
+      mma_16816(s, ku[0][i].x, ku[1][i].x, ku[0][i].y, ku[1][i].y, qf[i][0], qf[i][1]);
+      mma_16816(s, ku[0][i].z, ku[1][i].z, ku[0][i].w, ku[1][i].w, qf[i][2], qf[i][3]);
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      s[e] = kCap ? soft_cap(s[e], a.cap) : s[e] * a.scale_log2;
+      if (base + g + 8 * (e >> 1) >= k1) s[e] = -INFINITY;
+    }
+    float n0 = fmaxf(s[0], s[2]), n1 = fmaxf(s[1], s[3]);
+#pragma unroll
+    for (int off = 4; off < 32; off <<= 1) {
+      n0 = fmaxf(n0, __shfl_xor_sync(0xffffffffu, n0, off));
+      n1 = fmaxf(n1, __shfl_xor_sync(0xffffffffu, n1, off));
+    }
+    n0 = fmaxf(m0, n0);
+    n1 = fmaxf(m1, n1);
+    const float r0 = n0 == -INFINITY ? 0.f : n0, r1 = n1 == -INFINITY ? 0.f : n1;
+    const float f0 = exp2f(m0 - r0), f1 = exp2f(m1 - r1);
+    m0 = n0;
+    m1 = n1;
+    const float p0 = exp2f(s[0] - r0), p1 = exp2f(s[1] - r1), p2 = exp2f(s[2] - r0), p3 = exp2f(s[3] - r1);
+    l0 = fmaf(l0, f0, p0 + p2);
+    l1 = fmaf(l1, f1, p1 + p3);
+    const uint32_t h01 = pack_bf16x2(p0, p1), h23 = pack_bf16x2(p2, p3);
+    const float2 b01 = unpack_bf16x2(h01), b23 = unpack_bf16x2(h23);
+    const uint32_t hi0 = transpose_8x8(h01), hi1 = transpose_8x8(h23);
+    const uint32_t lo0 = transpose_8x8(pack_bf16x2(p0 - b01.x, p1 - b01.y)), lo1 = transpose_8x8(pack_bf16x2(p2 - b23.x, p3 - b23.y));
+#pragma unroll
+    for (int u = 0; u < VS; ++u) {
+      const uint32_t w[4][4] = {{vu[0][u].x, vu[0][u].y, vu[0][u].z, vu[0][u].w}, {vu[1][u].x, vu[1][u].y, vu[1][u].z, vu[1][u].w},
+                                {vu[2][u].x, vu[2][u].y, vu[2][u].z, vu[2][u].w}, {vu[3][u].x, vu[3][u].y, vu[3][u].z, vu[3][u].w}};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {   // features 64 u + 8 g + 2 j (row g) and + 1 (row g + 8)
+        const uint32_t a0 = __byte_perm(w[0][j], w[1][j], 0x5410), a1 = __byte_perm(w[0][j], w[1][j], 0x7632);
+        const uint32_t a2 = __byte_perm(w[2][j], w[3][j], 0x5410), a3 = __byte_perm(w[2][j], w[3][j], 0x7632);
+        o[u][j][0] *= f0;
+        o[u][j][1] *= f1;
+        o[u][j][2] *= f0;
+        o[u][j][3] *= f1;
+        mma_16816(o[u][j], a0, a1, a2, a3, lo0, lo1);
+        mma_16816(o[u][j], a0, a1, a2, a3, hi0, hi1);
+      }
     }
   }
+#pragma unroll
+  for (int off = 4; off < 32; off <<= 1) {
+    l0 += __shfl_xor_sync(0xffffffffu, l0, off);
+    l1 += __shfl_xor_sync(0xffffffffu, l1, off);
+  }
+  if (2 * t < G) {
+#pragma unroll
+    for (int u = 0; u < VS; ++u)
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) sm_o[warp][2 * t + (e & 1)][64 * u + 8 * g + 2 * j + (e >> 1)] = o[u][j][e];
+    if (g == 0) {
+      sm_m[warp][2 * t] = m0;
+      sm_m[warp][2 * t + 1] = m1;
+      sm_l[warp][2 * t] = l0;
+      sm_l[warp][2 * t + 1] = l1;
+    }
+  }
+  __syncthreads();
+  merge_warps<DV, G>(a, sm_o, sm_m, sm_l, b, hkv, split, n_splits);
 }
 
 // out[b, h, :] = sum_s part_o[s] 2^(m_s - M) / (sum_s l_s 2^(m_s - M) + the sink's weight); one CTA per (head, sequence). The
@@ -267,8 +427,12 @@ cudaError_t decode_launch(const DecArgs& a, int B, int n_splits, __nv_bfloat16* 
   const bool cap = a.cap.out > 0.f;
   if (n_splits > kMaxSplits || (a.pool > 0 && cap)) return cudaErrorInvalidValue;
   dim3 grid(n_splits, a.Hkv, B);
-  if (a.pool > 0) attn_decode_split_kernel<D, DV, G, false, true><<<grid, kDecWarps * 32, 0, stream>>>(a);
-  else if (cap) attn_decode_split_kernel<D, DV, G, true, false><<<grid, kDecWarps * 32, 0, stream>>>(a);
+  if (a.pool > 0) {
+    attn_decode_split_kernel<D, DV, G, false, true><<<grid, kDecWarps * 32, 0, stream>>>(a);
+  } else if constexpr (G >= 4) {   // one or two queries leave the columns of the matrix instructions empty and the scores cheap
+    if (cap) attn_decode_mma_kernel<D, DV, G, true><<<grid, kDecWarps * 32, 0, stream>>>(a);
+    else attn_decode_mma_kernel<D, DV, G, false><<<grid, kDecWarps * 32, 0, stream>>>(a);
+  } else if (cap) attn_decode_split_kernel<D, DV, G, true, false><<<grid, kDecWarps * 32, 0, stream>>>(a);
   else attn_decode_split_kernel<D, DV, G, false, false><<<grid, kDecWarps * 32, 0, stream>>>(a);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;

@@ -125,3 +125,36 @@ def test_gqa_layer_cached_paths_match_uncached(cuda_device):
         c, _, _ = gqa_attention(x[:, 199:], p, Hq, Hkv, dh, rope, 16, ck, cv, 199)
     got = torch.cat([a, b, c], dim=1)
     assert _rel_err(got, full) < 2e-2
+
+
+@pytest.mark.parametrize("D,Dv,H,Hkv", [(64, 64, 8, 2), (128, 128, 16, 2), (256, 256, 8, 1), (64, 128, 8, 1), (128, 256, 8, 2)])
+@pytest.mark.parametrize("window,keep,cap", [(0, 0, 0.0), (40, 5, 0.0), (0, 0, 20.0)])
+def test_decode_of_shared_kv_heads(cuda_device, D, Dv, H, Hkv, window, keep, cap):
+    """Four and eight queries per kv head over paged caches whose lengths surround the 16 keys of a step and the 64 of a block's round,
+    with more key ranges than keys; windows with kept first keys, capped scores with a sink. Probabilities are exact to 2^-17, so the
+    output differs by its own rounding to bf16, 2^-9."""
+    from jax_gpt_b200.ops.attention import attention_decode_paged
+    g = torch.Generator(device=cuda_device).manual_seed(29)
+    rnd = lambda *s: torch.randn(*s, device=cuda_device, generator=g)
+    lens, ps = [1, 15, 16, 17, 63, 64, 65, 127, 1000], 24
+    per = (max(lens) + ps - 1) // ps
+    pool = rnd(len(lens) * per + 1, ps, Hkv * (D + Dv)).to(torch.bfloat16)
+    pool[-1] = float("nan")                                        # a page that belongs to nobody
+    table = torch.randperm(len(lens) * per, device=cuda_device, generator=g).to(torch.int32).view(len(lens), per)
+    q, sink = rnd(len(lens), H, D).to(torch.bfloat16), rnd(H) if cap else None
+    ids = torch.arange(len(lens), device=cuda_device, dtype=torch.int32)
+    committed = torch.tensor(lens, device=cuda_device, dtype=torch.int32) - 1
+    out = attention_decode_paged(q, pool, table, ids, committed, Hkv, v_dim=Dv, window=window, keep_first=keep, softcap=cap, sink=sink)
+    for b, n in enumerate(lens):
+        pos = torch.arange(n, device=cuda_device)
+        rows = pool[table[b, pos // ps].long(), pos % ps].float()
+        k = rows[:, :Hkv * D].reshape(n, Hkv, D).repeat_interleave(H // Hkv, 1)
+        v = rows[:, Hkv * D:].reshape(n, Hkv, Dv).repeat_interleave(H // Hkv, 1)
+        sc = torch.einsum("hd,nhd->hn", q[b].float(), k) * D ** -0.5
+        if cap:
+            sc = torch.cat([cap * torch.tanh(sc / cap), sink[:, None]], 1)
+        if window:
+            sc = sc.masked_fill((pos < n - window) & (pos >= keep), float("-inf"))
+        ref = torch.einsum("hn,nhd->hd", torch.softmax(sc, -1)[:, :n], v)
+        rel = ((out[b].float() - ref).norm() / ref.norm()).item()
+        assert rel < 4e-3, (n, rel)
