@@ -17,11 +17,11 @@ from __future__ import annotations
 from typing import List, Optional
 
 import torch
-import torch.nn.functional as F
 
 from ... import _ext
 from ...cache.paged import PagedCache
 from ...ops.gemm import linear
+from ...ops.layer_tail import argmax_rows, layer_tail, silu_mul, tail_ok
 from ...ops.router import deepseek_router
 from ..qwen35.block import _slice
 from ..qwen35.primitives import precompute_rope_freqs
@@ -80,20 +80,31 @@ class DeepSeekV3DecodeEngine:
         return linear(o, ap["o_proj"])
 
     def _ffn(self, h, lp, is_moe: bool):
+        """(output, fp32 sum of the routed experts that belongs to it or None)."""
         c = self.c
         if not is_moe:
             m = lp["mlp"]
-            return linear(F.silu(linear(h, m["gate_proj"])) * linear(h, m["up_proj"]), m["down_proj"])
+            return linear(silu_mul(linear(h, m["gate_proj"]), linear(h, m["up_proj"])), m["down_proj"]), None
         mp = lp["moe"]
         w, idx = deepseek_router(h, mp["gate_weight"], mp["e_score_correction_bias"], c.n_experts_per_token, c.n_group,
                                  c.topk_group, c.routed_scaling_factor, c.norm_topk_prob)
-        if self.ep is not None:
-            routed = self.ep.forward(h, w, idx, mp).to(h.dtype)
+        if hasattr(self.ep, "routed_f32"):
+            routed = self.ep.routed_f32(h, w, idx, mp)
+        elif self.ep is not None:
+            routed = self.ep.forward(h, w, idx, mp).float()
         else:
             from ..qwen35.moe import expert_forward_single
-            routed = expert_forward_single(h, w, idx, mp)
-        shared = linear(F.silu(linear(h, mp["shared_gate_proj"])) * linear(h, mp["shared_up_proj"]), mp["shared_down_proj"])
-        return routed + shared
+            routed = expert_forward_single(h, w, idx, mp).float()
+        shared = linear(silu_mul(linear(h, mp["shared_gate_proj"]), linear(h, mp["shared_up_proj"])), mp["shared_down_proj"])
+        return shared, routed
+
+    def _add_norm(self, x, y, norm_w, routed=None):
+        """x + y + routed (fp32) and the norm of the sum."""
+        eps = self.c.rms_norm_eps
+        if tail_ok(x, y, norm_w):
+            return layer_tail(x, routed, y, norm_w=norm_w, eps=eps, one_plus=False)
+        x = x + (y if routed is None else (y + routed.to(y.dtype)))
+        return x, rms_norm(x, norm_w, eps)
 
     def _token_step(self):
         c, p = self.c, self.p
@@ -103,15 +114,16 @@ class DeepSeekV3DecodeEngine:
         self._lens1.copy_(self.cache.seq_lens)
         self._lens1.index_add_(0, self.ids_long, torch.ones_like(self.ids_t))
         x = p["embed"][self.tokens]
-        li = 0
-        for name, is_moe, n in (("dense_layers", False, c.first_k_dense), ("moe_layers", True, c.n_moe_layers)):
-            for i in range(n):
-                lp = _slice(p[name], i)
-                x = x + self._attention(rms_norm(x, lp["attn_norm"], c.rms_norm_eps), lp["attn"], li, pos)
-                x = x + self._ffn(rms_norm(x, lp["ffn_norm"], c.rms_norm_eps), lp, is_moe)
-                li += 1
-        logits = linear(rms_norm(x, p["final_norm"], c.rms_norm_eps), p["lm_head"])
-        self.next_tokens.copy_(logits.argmax(-1))
+        layers = [(_slice(p[name], i), is_moe) for name, is_moe, n in (("dense_layers", False, c.first_k_dense),
+                                                                      ("moe_layers", True, c.n_moe_layers)) for i in range(n)]
+        norms = [lp["attn_norm"] for lp, _ in layers] + [p["final_norm"]]
+        h = rms_norm(x, norms[0], c.rms_norm_eps)
+        for li, (lp, is_moe) in enumerate(layers):
+            x, h = self._add_norm(x, self._attention(h, lp["attn"], li, pos), lp["ffn_norm"])
+            y, routed = self._ffn(h, lp, is_moe)
+            x, h = self._add_norm(x, y, norms[li + 1], routed)
+        logits = linear(h, p["lm_head"])
+        argmax_rows(logits, out=self.next_tokens)
         self.cache.seq_lens.copy_(self._lens1)           # the step's tokens are now part of the sequences
         return logits
 

@@ -25,13 +25,13 @@ import math
 from typing import List, Optional
 
 import torch
-import torch.nn.functional as F
 
 from ...cache.paged import PagedCache
 from ...ops import attention as attn_ops
 from ...ops import grouped_gemm
 from ...ops import norm as norm_ops
 from ...ops.gemm import linear
+from ...ops.layer_tail import layer_tail, silu_mul, tail_ok
 from ...ops.rope import mla_prompt_ok, mla_prompt_rope
 from ...utils.profiling import scope
 from ..qwen35.block import _slice
@@ -110,7 +110,8 @@ def route_tokens(x: torch.Tensor, gate_weight, bias, c: DeepSeekV3Config):
 
 
 def swiglu_mlp(x, gate, up, down):
-    return linear(F.silu(linear(x, gate)) * linear(x, up), down)
+    g, u = linear(x, gate), linear(x, up)
+    return linear(silu_mul(g.flatten(0, -2), u.flatten(0, -2)).unflatten(0, g.shape[:-1]), down)
 
 
 def moe_ffn(x: torch.Tensor, mp, c: DeepSeekV3Config, ep=None) -> torch.Tensor:
@@ -120,14 +121,18 @@ def moe_ffn(x: torch.Tensor, mp, c: DeepSeekV3Config, ep=None) -> torch.Tensor:
     with scope("moe_routing"):
         w, idx = route_tokens(xf, mp["gate_weight"], mp["e_score_correction_bias"], c)
     with scope("moe_experts"):
-        if ep is not None:
+        if hasattr(ep, "routed_f32") and tail_ok(xf) and not (torch.is_grad_enabled() and any(torch.is_tensor(t) and t.requires_grad for t in mp.values())):
+            routed = ep.routed_f32(xf, w, idx, mp)
+        elif ep is not None:
             routed = ep.forward(xf, w, idx, mp).to(x.dtype)
         else:
             from ..qwen35.moe import expert_forward_single
             routed = expert_forward_single(xf, w, idx, mp)
     with scope("moe_shared_expert"):
         shared = swiglu_mlp(xf, mp["shared_gate_proj"], mp["shared_up_proj"], mp["shared_down_proj"])
-    return (routed + shared).reshape(B, T, D)
+    if routed.dtype == torch.float32 and shared.dtype == torch.bfloat16 and tail_ok(shared):
+        return layer_tail(routed=routed, shared=shared).reshape(B, T, D)
+    return (routed.to(x.dtype) + shared).reshape(B, T, D)
 
 
 # ------------------------------------------------------------------------------------------------

@@ -9,7 +9,7 @@ from ...parallel.tp_ops import copy_to_tp, reduce_from_tp
 from ...utils.profiling import scope
 from .deltanet import deltanet_prefill, deltanet_recurrent_step
 from .gqa import gqa_attention
-from .moe import moe_layer
+from .moe import moe_residual
 from .primitives import rms_norm
 
 
@@ -55,8 +55,7 @@ def deltanet_layer_forward(x, lp, delta_M, delta_conv, config, is_decode: bool, 
         x = x + a
     with scope("deltanet_moe"):
         h = rms_norm(x, lp["moe_norm"], c.rms_norm_eps)
-        x = x + moe_layer(h, lp["moe"], c.n_experts_per_token, group=ep_group, n_experts=c.n_routed_experts,
-                          tp_group=tp_group)
+        x = moe_residual(x, h, lp["moe"], c.n_experts_per_token, group=ep_group, n_experts=c.n_routed_experts, tp_group=tp_group)
     return x, M, conv
 
 
@@ -70,8 +69,7 @@ def gqa_layer_forward(x, lp, cache_k, cache_v, cache_pos, config, rope_freqs, ep
         x = x + a
     with scope("gqa_moe"):
         h = rms_norm(x, lp["moe_norm"], c.rms_norm_eps)
-        x = x + moe_layer(h, lp["moe"], c.n_experts_per_token, group=ep_group, n_experts=c.n_routed_experts,
-                          tp_group=tp_group)
+        x = moe_residual(x, h, lp["moe"], c.n_experts_per_token, group=ep_group, n_experts=c.n_routed_experts, tp_group=tp_group)
     return x, nk, nv
 
 

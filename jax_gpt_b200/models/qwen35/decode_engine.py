@@ -28,13 +28,15 @@ from typing import Optional
 import torch
 
 from ...ops import attention as attn_ops
+from ...ops.layer_tail import argmax_rows, gate_heads, layer_tail, tail_ok
+from ...ops.rope import rmsnorm_rope
 from .block import _slice
 from .cache import HybridCache
 from .config import Qwen35Config
 from .deltanet import deltanet_recurrent_step
 from .fp8 import matmul_maybe_fp8
-from .moe import moe_layer
-from .primitives import apply_rotary_emb, precompute_rope_freqs, rms_norm
+from .moe import fused_tail_ok, moe_layer, moe_parts
+from .primitives import precompute_rope_freqs, rms_norm
 
 
 class Qwen35DecodeEngine:
@@ -124,28 +126,37 @@ class Qwen35DecodeEngine:
             layers.append((delta, gl))
         return layers
 
-    # ---- layers (x is (B, D)) -------------------------------------------------------------------------
-    def _moe(self, x, lp):
-        c = self.c
-        h = rms_norm(x, lp["moe_norm"], c.rms_norm_eps)
-        return x + moe_layer(h[:, None, :], lp["moe"], c.n_experts_per_token, group=self.ep,
-                             n_experts=c.n_routed_experts)[:, 0]
+    # ---- layers (x is (B, D), h its norm for the layer at hand) -----------------------------------------
+    def _add_norm(self, x, y, norm_w):
+        """x + y and the norm of the sum."""
+        if tail_ok(x, y, norm_w):
+            return layer_tail(x, shared=y, norm_w=norm_w, eps=self.c.rms_norm_eps)
+        x = x + y
+        return x, rms_norm(x, norm_w, self.c.rms_norm_eps)
 
-    def _delta_layer(self, x, lp, gi: int, i: int):
+    def _mixed(self, x, a, lp, next_norm):
+        """The mixer's output ``a`` is added, then the expert layer runs: the new x and its norm by ``next_norm``."""
+        c, moe = self.c, lp["moe"]
+        x, h = self._add_norm(x, a, lp["moe_norm"])
+        if fused_tail_ok(h, moe, self.ep) and tail_ok(x, next_norm):
+            routed, shared = moe_parts(h, moe, c.n_experts_per_token, self.ep)
+            return layer_tail(x, routed, shared, h, moe["shared_expert_gate_weight"], next_norm, c.rms_norm_eps)
+        y = moe_layer(h[:, None, :], moe, c.n_experts_per_token, group=self.ep, n_experts=c.n_routed_experts)[:, 0]
+        return self._add_norm(x, y, next_norm)
+
+    def _delta_layer(self, x, h, lp, gi: int, i: int, next_norm):
         c = self.c
-        h = rms_norm(x, lp["attn_norm"], c.rms_norm_eps)
         state, conv = self.M[gi, i], self.conv[gi, i]
         a, new_state, new_conv = deltanet_recurrent_step(h[:, None, :], lp["attn"], state, conv, c.delta_n_qk_heads,
                                                          c.delta_n_v_heads, c.delta_qk_head_dim, c.delta_v_head_dim)
         if new_state.data_ptr() != state.data_ptr():         # library path returns new tensors; the kernel works in place
             state.copy_(new_state)
             conv.copy_(new_conv)
-        return self._moe(x + a[:, 0], lp)
+        return self._mixed(x, a[:, 0], lp, next_norm)
 
-    def _gqa_layer(self, x, lp, gi: int):
+    def _gqa_layer(self, x, h, lp, gi: int, next_norm):
         c, ap = self.c, lp["attn"]
         B, Hq, Hkv, dh = self.B, c.gqa_n_q_heads, c.gqa_n_kv_heads, c.gqa_head_dim
-        h = rms_norm(x, lp["attn_norm"], c.rms_norm_eps)
         if "qkv_proj" in ap:
             qkv = matmul_maybe_fp8(h, ap["qkv_proj"])
             nq, nk = 2 * Hq * dh, Hkv * dh
@@ -156,10 +167,8 @@ class Qwen35DecodeEngine:
             qg = matmul_maybe_fp8(h, ap["q_proj"]).reshape(B, 1, Hq, 2 * dh)
             k = matmul_maybe_fp8(h, ap["k_proj"]).reshape(B, 1, Hkv, dh)
             v = matmul_maybe_fp8(h, ap["v_proj"]).reshape(B, 1, Hkv, dh)
-        q, gate = qg[..., :dh], qg[..., dh:]
         fr = self.rope.index_select(0, self.pos_t)                                   # (1, rope_dim/2, 2)
-        q = apply_rotary_emb(rms_norm(q.contiguous(), ap["q_norm"]), fr, c.gqa_rope_dim)
-        k = apply_rotary_emb(rms_norm(k.contiguous(), ap["k_norm"]), fr, c.gqa_rope_dim)
+        q, k = rmsnorm_rope(qg[..., :dh], ap["q_norm"], fr, c.gqa_rope_dim), rmsnorm_rope(k, ap["k_norm"], fr, c.gqa_rope_dim)
         if self.paged is not None:
             pc = self.paged
             row = torch.cat([k.reshape(B, 1, Hkv * dh), v.reshape(B, 1, Hkv * dh)], dim=-1).to(pc.pool.dtype)
@@ -177,18 +186,22 @@ class Qwen35DecodeEngine:
             ck.index_copy_(2, self.pos_t, k.permute(0, 2, 1, 3).to(ck.dtype))
             cv.index_copy_(2, self.pos_t, v.permute(0, 2, 1, 3).to(cv.dtype))
             o = attn_ops.attention_decode(q.reshape(B, Hq, dh), ck, cv, pos=self.pos_i32, scratch=self.dec_scratch)
-        o = (o.float() * torch.sigmoid(gate[:, 0].float())).to(x.dtype)
-        return self._moe(x + matmul_maybe_fp8(o.reshape(B, Hq * dh), ap["o_proj"]), lp)
+        o = gate_heads(o.reshape(B, Hq, dh), qg[:, 0]).reshape(B, Hq * dh)
+        return self._mixed(x, matmul_maybe_fp8(o, ap["o_proj"]), lp, next_norm)
 
     def _token_step(self):
         c, p = self.c, self.p
         x = p["embed"][self.tokens]
+        norms = [lp["attn_norm"] for delta, gqa in self._layers for lp in (*delta, gqa)] + [p["final_norm"]]
+        h, at = rms_norm(x, norms[0], c.rms_norm_eps), 1
         for gi, (delta, gqa) in enumerate(self._layers):
             for i, lp in enumerate(delta):
-                x = self._delta_layer(x, lp, gi, i)
-            x = self._gqa_layer(x, gqa, gi)
-        logits = matmul_maybe_fp8(rms_norm(x, p["final_norm"], c.rms_norm_eps), p["lm_head"])
-        self.next_tokens.copy_(logits.argmax(-1))
+                x, h = self._delta_layer(x, h, lp, gi, i, norms[at])
+                at += 1
+            x, h = self._gqa_layer(x, h, gqa, gi, norms[at])
+            at += 1
+        logits = matmul_maybe_fp8(h, p["lm_head"])
+        argmax_rows(logits, out=self.next_tokens)
         self.pos_t.add_(1)
         self.pos_i32.add_(1)
         if self.paged is not None:

@@ -9,6 +9,7 @@ from typing import Optional
 import torch
 
 from ...ops import attention as attn_ops
+from ...ops.layer_tail import gate_heads
 from .fp8 import matmul_maybe_fp8
 from .primitives import apply_rotary_emb, rms_norm
 
@@ -38,7 +39,7 @@ def gqa_attention(x, params, n_q_heads: int, n_kv_heads: int, head_dim: int, rop
         kv_lo = (tp_rank(tp_group) * n_q_heads) // g
         n_kv_heads = max(1, n_q_heads // g)
     qg = matmul_maybe_fp8(copy_to_tp(x, tp_group) if sharded else x, params["q_proj"]).reshape(B, T, n_q_heads, 2 * head_dim)
-    q, gate = qg[..., :head_dim], qg[..., head_dim:]
+    q = qg[..., :head_dim]
     k = matmul_maybe_fp8(x, params["k_proj"]).reshape(B, T, hkv_all, head_dim)
     v = matmul_maybe_fp8(x, params["v_proj"]).reshape(B, T, hkv_all, head_dim)
     pos = int(cache_pos) if cache_pos is not None else 0
@@ -78,7 +79,7 @@ def gqa_attention(x, params, n_q_heads: int, n_kv_heads: int, head_dim: int, rop
             out = attn_ops.attention_cached(q.contiguous(), cache_k, cache_v, pos + T, pos)
     else:
         out = attn_ops.attention(q.contiguous(), k.contiguous(), v.contiguous(), causal=True)
-    out = out * torch.sigmoid(gate.float()).to(out.dtype)
+    out = gate_heads(out, qg)
     y = matmul_maybe_fp8(out.reshape(B, T, n_q_heads * head_dim), params["o_proj"])
     if sharded:
         return reduce_from_tp(y, tp_group), full_k, full_v

@@ -15,7 +15,6 @@ from __future__ import annotations
 from typing import Optional
 
 import torch
-import torch.nn.functional as F
 
 from .fp8 import dequantize_weight, is_fp8_weight, matmul_maybe_fp8
 
@@ -120,13 +119,28 @@ def expert_forward_tp(x: torch.Tensor, weights: torch.Tensor, idx: torch.Tensor,
 
 
 def shared_expert_forward(x: torch.Tensor, params) -> torch.Tensor:
+    from ...ops.layer_tail import silu_mul
     if "shared_gate_up_proj" in params:       # gate | up as one GEMM over concatenated weights (decode engine)
-        gu = matmul_maybe_fp8(x, params["shared_gate_up_proj"])
-        half = gu.shape[-1] // 2
-        return matmul_maybe_fp8(F.silu(gu[..., :half]) * gu[..., half:], params["shared_down_proj"])
-    g = matmul_maybe_fp8(x, params["shared_gate_proj"])
-    u = matmul_maybe_fp8(x, params["shared_up_proj"])
-    return matmul_maybe_fp8(F.silu(g) * u, params["shared_down_proj"])
+        g, u = matmul_maybe_fp8(x, params["shared_gate_up_proj"]).chunk(2, -1)
+    else:
+        g, u = matmul_maybe_fp8(x, params["shared_gate_proj"]), matmul_maybe_fp8(x, params["shared_up_proj"])
+    return matmul_maybe_fp8(silu_mul(g, u), params["shared_down_proj"])
+
+
+def fused_tail_ok(x, params, group) -> bool:
+    """Inference on the one-kernel expert path with plain bf16 shared-expert weights: the layer's end is one launch."""
+    from ...ops.layer_tail import tail_ok
+    return (hasattr(group, "routed_f32") and tail_ok(x, params["shared_expert_gate_weight"]) and torch.is_tensor(params["gate_weight"])
+            and not (torch.is_grad_enabled() and any(torch.is_tensor(t) and t.requires_grad for t in params.values())))
+
+
+def moe_parts(x: torch.Tensor, params, k: int, group):
+    """x (M, D) -> (routed fp32, in the expert kernel's buffer, shared): what ``layer_tail`` adds up."""
+    from ...ops.gemm import linear_f32out
+    from ...ops.router import softmax_topk_ids32
+    w, idx = softmax_topk_ids32(linear_f32out(x, params["gate_weight"]), k)
+    routed = group.routed_f32(x, w, idx, params)
+    return routed, shared_expert_forward(x, params)
 
 
 def moe_layer(x: torch.Tensor, params, n_experts_per_token: int, n_devices: int = 1, axis_name: str = "tp",
@@ -139,6 +153,10 @@ def moe_layer(x: torch.Tensor, params, n_experts_per_token: int, n_devices: int 
     the experts among them (partial outputs summed over the group)."""
     B, T, D = x.shape
     xf = x.reshape(B * T, D)
+    if fused_tail_ok(xf, params, group):
+        from ...ops.layer_tail import layer_tail
+        routed, shared = moe_parts(xf, params, n_experts_per_token, group)
+        return layer_tail(routed=routed, shared=shared, h=xf, gate_w=params["shared_expert_gate_weight"]).reshape(B, T, D)
     w, idx = moe_routing(xf, params["gate_weight"], n_experts_per_token)
     if callable(group):
         grads = {n: params.get(n + "@grad") for n in ("gate_proj", "up_proj", "down_proj")}
@@ -154,3 +172,15 @@ def moe_layer(x: torch.Tensor, params, n_experts_per_token: int, n_devices: int 
     shared = shared_expert_forward(xf, params)
     sg = torch.sigmoid(matmul_maybe_fp8(xf, params["shared_expert_gate_weight"]).float()).to(x.dtype)
     return (routed + shared * sg).reshape(B, T, D)
+
+
+def moe_residual(x: torch.Tensor, h: torch.Tensor, params, n_experts_per_token: int, group=None, n_experts: Optional[int] = None,
+                 tp_group=None) -> torch.Tensor:
+    """``x + moe_layer(h)``, the sum part of the layer's last launch where that exists."""
+    xf, hf = x.reshape(-1, x.shape[-1]), h.reshape(-1, h.shape[-1])
+    if fused_tail_ok(hf, params, group):
+        from ...ops.layer_tail import layer_tail, tail_ok
+        if tail_ok(xf):
+            routed, shared = moe_parts(hf, params, n_experts_per_token, group)
+            return layer_tail(xf, routed, shared, hf, params["shared_expert_gate_weight"]).reshape(x.shape)
+    return x + moe_layer(h, params, n_experts_per_token, group=group, n_experts=n_experts, tp_group=tp_group)

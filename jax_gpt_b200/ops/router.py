@@ -39,6 +39,14 @@ def softmax_topk_router(logits: torch.Tensor, k: int):
     return w / w.sum(-1, keepdim=True), idx
 
 
+def softmax_topk_ids32(logits: torch.Tensor, k: int):
+    """``softmax_topk_router`` for inference, with int32 ids (what the expert kernels read)."""
+    if _cuda_ok(logits, k):
+        return router_cuda(0, logits, None, k)
+    w, idx = softmax_topk_router(logits, k)
+    return w, idx.to(torch.int32)
+
+
 def deepseek_router_from_logits(logits: torch.Tensor, bias: torch.Tensor, k: int, n_group: int, topk_group: int,
                                 scale: float, norm_topk: bool = True):
     M, E = logits.shape

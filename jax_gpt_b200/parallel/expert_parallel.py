@@ -293,9 +293,13 @@ class EPMoEInferenceRuntime:
     def forward(self, x, weights, idx, params, grads=None):
         """``grads`` is accepted (and ignored) so that the object also fits the callable form
         ``group(x, weights, idx, params, grads)`` of models/qwen35/moe.py:moe_layer."""
-        return self._layer(x.shape[0]).forward(x.contiguous(), weights, idx, params).to(x.dtype)
+        return self.routed_f32(x, weights, idx, params).to(x.dtype)
 
     __call__ = forward
+
+    def routed_f32(self, x, weights, idx, params):
+        """The experts' sum in fp32, in the kernel's own buffer: the next call with as many tokens overwrites it."""
+        return self._layer(x.shape[0]).forward(x.contiguous(), weights, idx, params)
 
 
 def quantize_stacked_experts_fp8(moe_params: dict) -> dict:

@@ -253,6 +253,41 @@ def test_mla_rope_layout_kernels(cuda_device, B, T, H, dn, dr, dv, kvr):
     assert near(rows, torch.cat([c_kv.view(n, -1), turn(kv.view(n, -1)[:, kvr:])[:, 0]], -1))
 
 
+@pytest.mark.parametrize("M,D", [(1, 8), (3, 2048), (33, 2056), (5, 7168), (2, 8192)])
+def test_layer_tail(cuda_device, M, D):
+    """Every combination of parts that callers use vs the same sums in fp32 torch. One rounding to bf16 (2^-9 of the value) on top of
+    fp32 sums; the norm is of the rounded row, so a row that rounds the other way moves it by a bf16 step."""
+    from jax_gpt_b200.ops import layer_tail as L
+    g = torch.Generator(device=cuda_device).manual_seed(13)
+    rnd = lambda *s: torch.randn(*s, device=cuda_device, generator=g)
+    bf = lambda *s: rnd(*s).to(torch.bfloat16)
+    x, routed, shared, h, gate, norm = bf(M, D), rnd(M, D), bf(M, D), bf(M, D), bf(D, 1) * D ** -0.5, bf(D)
+    for kw in (dict(x=x, shared=shared), dict(routed=routed, shared=shared, h=h, gate_w=gate), dict(x=x, routed=routed, shared=shared),
+               dict(x=x, routed=routed, shared=shared, h=h, gate_w=gate, norm_w=norm), dict(x=x, shared=shared, norm_w=norm, one_plus=False, eps=1e-5)):
+        got, want = L.layer_tail(**kw), L.layer_tail_ref(**kw)
+        for a, b in zip(got if isinstance(got, tuple) else (got,), want if isinstance(want, tuple) else (want,)):
+            assert _rel(a, b) < 4e-3 and torch.isfinite(a).all()
+    assert not L.tail_ok(x.requires_grad_()) and L.tail_ok(shared)
+
+
+@pytest.mark.parametrize("rows,N,col", [(1, 1, 0), (2, 7, 0), (3, 1000, 1), (64, 129280, 0), (1, 151936, 0)])
+def test_argmax_rows(cuda_device, rows, N, col):
+    """Ties, both zeros, infinities and NaNs as torch orders them; rows that start off a 16-byte boundary."""
+    from jax_gpt_b200.ops.layer_tail import argmax_rows
+    g = torch.Generator(device=cuda_device).manual_seed(17)
+    x = torch.randn(rows, N + 8, device=cuda_device, generator=g).to(torch.bfloat16)[:, col:col + N]
+    first = lambda t: (t == t.amax(-1, keepdim=True)).float().argmax(-1) if not t.isnan().any() else t.isnan().float().argmax(-1)
+    assert torch.equal(argmax_rows(x), first(x))
+    for fill in (-float("inf"), -0.0, -3.0):
+        y = torch.full_like(x, fill)
+        y[:, N // 2:] = 0.0 if fill == 0 else fill
+        assert torch.equal(argmax_rows(y), torch.zeros(rows, device=cuda_device, dtype=torch.long))
+    x[:, N // 3] = float("inf")
+    assert (argmax_rows(x) == N // 3).all()
+    x[:, 2 * N // 3:] = float("nan")
+    assert (argmax_rows(x) == 2 * N // 3).all()
+
+
 @pytest.mark.parametrize("M,N,K", [(300, 512, 1024), (256, 384, 512), (1024, 2048, 7168)])
 def test_mxfp8_gemm_hardware_block_scales(cuda_device, M, N, K):
     """tcgen05 block-scaled MMA (UE8M0 scales in TMEM) vs the de-quantised fp32 product."""
