@@ -1,6 +1,7 @@
 // The end of a layer and of a token step as single launches. A decode step of few sequences is a chain of small kernels of which each
 // costs 1.5 - 2 us whatever it does: the sum of residual, routed and gated shared expert with the norm that follows took nine
-// (cast, gate product, cast, sigmoid, cast, product, two sums, norm), the greedy choice two.
+// (cast, gate product, cast, sigmoid, cast, product, two sums, norm), the expert bookkeeping three (clear, count, clear), the greedy
+// choice two.
 #include "layer_tail.cuh"
 
 #include "common.cuh"
@@ -102,6 +103,48 @@ __global__ void __launch_bounds__(256) layer_tail_kernel(const LayerTailArgs a) 
   }
 }
 
+// Block 0 counts in shared memory, the others clear the output.
+__global__ void __launch_bounds__(512)
+moe_prepare_zero_kernel(const int* __restrict__ idx, int n_pairs, int n_experts, int* __restrict__ counts, int* __restrict__ pos,
+                        float4* __restrict__ out, int64_t n_out4, int* __restrict__ order, int* __restrict__ flags, int n_flags) {
+  __shared__ int cnt[kPrepareMaxExperts], sums[16];
+  if (blockIdx.x > 0) {
+    const int64_t step = static_cast<int64_t>(gridDim.x - 1) * blockDim.x;
+    for (int64_t i = static_cast<int64_t>(blockIdx.x - 1) * blockDim.x + threadIdx.x; i < n_out4; i += step)
+      out[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    return;
+  }
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  cnt[t] = 0;
+  __syncthreads();
+  for (int p = t; p < n_pairs; p += 512) {
+    const int e = idx[p];
+    pos[p] = e >= 0 && e < n_experts ? atomicAdd(&cnt[e], 1) : 0;
+  }
+  if (order != nullptr)
+    for (int i = t; i < n_flags; i += 512) flags[i] = 0;
+  __syncthreads();
+  const int mine = cnt[t];
+  if (t < n_experts) counts[t] = mine;
+  if (order == nullptr) return;
+  int incl = mine;              // first place of every expert
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int n = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += n;
+  }
+  if (lane == 31) sums[warp] = incl;
+  __syncthreads();
+  int first = incl - mine;
+  for (int w = 0; w < warp; ++w) first += sums[w];
+  cnt[t] = first;
+  __syncthreads();
+  for (int p = t; p < n_pairs; p += 512) {
+    const int e = idx[p];
+    if (e >= 0 && e < n_experts) order[cnt[e] + pos[p]] = p;
+  }
+}
+
 __global__ void __launch_bounds__(256)
 silu_mul_kernel(const __nv_bfloat16* __restrict__ g, int64_t ldg, const __nv_bfloat16* __restrict__ u, int64_t ldu,
                 __nv_bfloat16* __restrict__ out, int64_t n8, int i8) {
@@ -198,6 +241,17 @@ cudaError_t launch_layer_tail(const LayerTailArgs& a, cudaStream_t st) {
   if (a.D <= 2048) layer_tail_kernel<1><<<a.rows, 256, 0, st>>>(a);
   else if (a.D <= 4096) layer_tail_kernel<2><<<a.rows, 256, 0, st>>>(a);
   else layer_tail_kernel<4><<<a.rows, 256, 0, st>>>(a);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_moe_prepare_zero(const int* idx, int n_pairs, int n_experts, int* counts, int* pos, float* out, int64_t n_out,
+                                    int* order, int* flags, int n_flags, cudaStream_t st) {
+  if ((order != nullptr && flags == nullptr) || n_pairs < 0 || n_pairs > kPrepareMaxPairs || n_experts < 1 || n_experts > kPrepareMaxExperts || n_out % 4 != 0)
+    return cudaErrorInvalidValue;
+  const int64_t want = (n_out / 4 + 2047) / 2048;       // four stores a thread
+  moe_prepare_zero_kernel<<<1 + static_cast<int>(want < 1184 ? want : 1184), 512, 0, st>>>(idx, n_pairs, n_experts, counts, pos,
+                                                                                       reinterpret_cast<float4*>(out), n_out / 4, order,
+                                                                                       flags, n_flags);
   return cudaGetLastError();
 }
 

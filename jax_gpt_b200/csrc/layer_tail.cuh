@@ -27,6 +27,13 @@ struct LayerTailArgs {
 };
 cudaError_t launch_layer_tail(const LayerTailArgs& a, cudaStream_t stream);
 
+// counts[e] = pairs of expert e, pos[p] = rank of pair p among its expert's, out[0 .. n_out) = 0, in one launch. At most
+// kPrepareMaxPairs pairs and kPrepareMaxExperts experts; n_out a multiple of 4 on a 16-byte boundary.
+// With `order`: the pairs sorted by expert, and `flags` [n_flags] cleared (what the expert kernel of one rank starts from).
+constexpr int kPrepareMaxPairs = 8192, kPrepareMaxExperts = 512;
+cudaError_t launch_moe_prepare_zero(const int* idx, int n_pairs, int n_experts, int* counts, int* pos, float* out, int64_t n_out,
+                                    int* order, int* flags, int n_flags, cudaStream_t stream);
+
 // out = silu(g) * u, rounded once; rows of I features (a multiple of 8), g and u with row strides (multiples of 8), out contiguous; all
 // on 16-byte boundaries.
 cudaError_t launch_silu_mul(const __nv_bfloat16* g, int64_t ldg, const __nv_bfloat16* u, int64_t ldu, __nv_bfloat16* out, int64_t rows,

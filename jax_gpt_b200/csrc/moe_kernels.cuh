@@ -39,8 +39,8 @@ struct EpMoeArgs {
   __nv_bfloat16* act;       // [cap_rows, inter] SwiGLU output
   __nv_bfloat16* gu;        // [cap_rows, 2 * inter] gate | up pre-activations saved for backward, or nullptr
   unsigned* arrive_target;  // [e_local] arrivals expected once this launch's rows are in (cumulative)
-  int* act_ready;           // [cap_rows / 128 + e_local + 1] per m-tile count of finished GEMM1 epilogue warps, then the
-                            // forward launch's tile counter
+  int* act_ready;           // [cap_rows / 128 + e_local + 2] per m-tile count of finished GEMM1 epilogue warps, then the
+                            // forward launch's tile counter and its count of finished blocks (one rank)
   int* slot_out;            // [tokens * top_k] bf16 forward: scratch, this rank's pair ids sorted by expert (the dispatch
                             // order); FP8 forward: row of each pair in its destination's receive buffer
   int* rows_out;            // [e_local] rows received per local expert (for the caller / backward)
@@ -59,6 +59,7 @@ struct EpMoeArgs {
   float* d_down;                               // [e_local, inter, d_model]
   uint64_t wait_budget_ns;
   int* status;
+  int prepared;  // forward on one rank: slot_out holds the order and act_ready is cleared (launch_moe_prepare_zero)
   long long* prof;  // set by the launchers: per-CTA phase timeline of this launch (kMoeProfFields per CTA), or nullptr
 };
 

@@ -51,7 +51,7 @@ class FusedEPMoE:
         self.out_acc = comm.alloc(tokens * d_model, torch.float32)
         self.act = torch.zeros(self.cap_rows, inter, device=dev, dtype=torch.bfloat16)
         self.arrive_target = torch.zeros(self.e_local, device=dev, dtype=torch.int32)
-        self.act_ready = torch.zeros(self.cap_rows // 128 + self.e_local + 1, device=dev, dtype=torch.int32)  # + tile counter
+        self.act_ready = torch.zeros(self.cap_rows // 128 + self.e_local + 2, device=dev, dtype=torch.int32)  # + tile and block counter
         self.slot_out = torch.zeros(tokens * top_k, device=dev, dtype=torch.int32)
         self.rows_out = torch.zeros(self.e_local, device=dev, dtype=torch.int32)
         self.my_counts = torch.zeros(n_experts, device=dev, dtype=torch.int32)
@@ -98,14 +98,14 @@ class FusedEPMoE:
         c = self.comm
         idx32 = idx.to(torch.int32).contiguous().view(-1)
         w32 = weights.to(torch.float32).contiguous().view(-1)
-        ops.moe_prepare(idx32, self.my_counts, self.pos)
+        alone = (self.slot_out, self.act_ready) if c.world == 1 else (None, None)
+        prepared = ops.moe_prepare_zero(idx32, self.my_counts, self.pos, self.out_acc.tensor, *alone)
         self.launch_token += 1
-        self.out_acc.tensor.zero_()
         ops.ep_moe_forward(c.world, c.rank, self.k, self.e_local, self.cap_rows, x.contiguous(), idx32, w32, self.pos,
                            self.my_counts, self.recv_x.peer_ptrs, self.recv_meta.peer_ptrs, self.recv_w.peer_ptrs,
                            self.counts_all.peer_ptrs, self.arrive.peer_ptrs, self.out_acc.peer_ptrs, c.ctrl.peer_ptrs,
                            self.act, self.arrive_target, self.act_ready, self.slot_out, self.rows_out,
-                           params["gate_proj"], params["up_proj"], params["down_proj"], c.wait_seconds, self.gu)
+                           params["gate_proj"], params["up_proj"], params["down_proj"], c.wait_seconds, self.gu, prepared)
         res = self.out_acc.tensor.view(self.tokens, self.D)
         if out is not None:
             out.copy_(res)
@@ -207,8 +207,7 @@ class FusedEPMoEFp8:
         c = self.comm
         idx32 = idx.to(torch.int32).contiguous().view(-1)
         w32 = weights.to(torch.float32).contiguous().view(-1)
-        ops.moe_prepare(idx32, self.my_counts, self.pos)
-        self.out_acc.tensor.zero_()
+        ops.moe_prepare_zero(idx32, self.my_counts, self.pos, self.out_acc.tensor)
         ops.ep_moe_forward_fp8(c.world, c.rank, self.k, self.e_local, self.cap_rows, x.contiguous(), idx32, w32, self.pos,
                                self.my_counts, self.xq, self.xe, self.recv_q.peer_ptrs, self.recv_sf.peer_ptrs,
                                self.recv_meta.peer_ptrs, self.recv_w.peer_ptrs, self.counts_all.peer_ptrs,

@@ -288,6 +288,25 @@ def test_argmax_rows(cuda_device, rows, N, col):
     assert (argmax_rows(x) == 2 * N // 3).all()
 
 
+@pytest.mark.parametrize("n_pairs,E,n_out", [(1, 8, 4), (10, 512, 2048), (8192, 512, 4096), (8200, 64, 1 << 20), (0, 32, 4), (640, 33, 6)])
+def test_moe_prepare_zero(cuda_device, n_pairs, E, n_out):
+    """Counts, a distinct rank per pair of an expert, a cleared output; below and above the one-launch sizes."""
+    from jax_gpt_b200 import _ext
+    g = torch.Generator(device=cuda_device).manual_seed(19)
+    idx = torch.randint(0, E, (n_pairs,), device=cuda_device, generator=g, dtype=torch.int32)
+    counts, pos, out = (torch.full((n,), 7, device=cuda_device, dtype=torch.int32) for n in (E, n_pairs, n_out))
+    out = out.float()
+    _ext.ops().moe_prepare_zero(idx, counts, pos, out)
+    assert torch.equal(counts.long(), torch.bincount(idx.long(), minlength=E)) and not out.any()
+    key = idx.long() * 100000 + pos
+    assert key.unique().numel() == n_pairs and (n_pairs == 0 or ((pos >= 0) & (pos < counts[idx.long()])).all())
+    order, flags = torch.full((n_pairs + 3,), -1, device=cuda_device, dtype=torch.int32), torch.ones(777, device=cuda_device, dtype=torch.int32)
+    if _ext.ops().moe_prepare_zero(idx, counts, pos, out, order, flags):
+        assert torch.equal(order[:n_pairs].long(), (idx.long() * 100000 + pos).argsort()) and (order[n_pairs:] == -1).all() and not flags.any()
+    else:
+        assert n_pairs > 8192 or n_out % 4
+
+
 @pytest.mark.parametrize("M,N,K", [(300, 512, 1024), (256, 384, 512), (1024, 2048, 7168)])
 def test_mxfp8_gemm_hardware_block_scales(cuda_device, M, N, K):
     """tcgen05 block-scaled MMA (UE8M0 scales in TMEM) vs the de-quantised fp32 product."""
