@@ -71,6 +71,7 @@ __global__ void __launch_bounds__(kBwd2Threads, 1)
 attn_bwd2_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                  const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tdo,
                  const __grid_constant__ Bwd2Args a) {
+  let_dependents_start();
   constexpr int D = kD;
   extern __shared__ __align__(1024) uint8_t smem[];
   if ((smem_u32(smem) & 1023u) != 0) {

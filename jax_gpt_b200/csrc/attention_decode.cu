@@ -387,6 +387,7 @@ template <int D>
 __global__ void __launch_bounds__(512)
 attn_decode_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml, int n_splits,
                          __nv_bfloat16* __restrict__ out, int64_t ldo, int H, const float* __restrict__ sink) {
+  let_dependents_start();
   constexpr int kGroups = 512 / D;
   __shared__ float wt[kMaxSplits], acc_s[kGroups][D], red[1];
   const int h = blockIdx.x, b = blockIdx.y, c = threadIdx.x % D, grp = threadIdx.x / D;

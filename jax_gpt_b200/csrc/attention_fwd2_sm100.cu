@@ -235,6 +235,7 @@ template <int D>
 __global__ void __launch_bounds__(kThreads2, 1)
 attn_fwd2_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                  const __grid_constant__ CUtensorMap tv, const __grid_constant__ Fwd2Args a) {
+  let_dependents_start();
   using C = Fwd2Cfg<D>;
   extern __shared__ __align__(1024) uint8_t smem[];
   if ((smem_u32(smem) & 1023u) != 0) {

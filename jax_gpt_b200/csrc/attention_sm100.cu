@@ -99,6 +99,7 @@ template <int D, int DV, int kMask, bool kCap>
 __global__ void __launch_bounds__(kThreads, (D == 64) ? 2 : 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                 const __grid_constant__ CUtensorMap tv, const __grid_constant__ FwdArgs a) {
+  let_dependents_start();
   using C = FwdCfg<D, DV>;
   constexpr bool kWindow = kMask != kAll;
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -684,6 +685,7 @@ template <int D>
 __global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ o, int64_t ldo,
                                   const __nv_bfloat16* __restrict__ dout, int64_t lddo, float* __restrict__ delta,
                                   int B, int T, int H) {
+  let_dependents_start();
   constexpr int kLanesPerHead = D / 8;   // 8 (D = 64) or 16 (D = 128): divides 32
   const int64_t row = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -709,6 +711,7 @@ __global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ o, int64_t l
 
 __global__ void cast_rows_kernel(const float* __restrict__ src, int64_t lds, __nv_bfloat16* __restrict__ dst,
                                  int64_t ldd, int M, int N) {
+  let_dependents_start();
   const int n4 = N / 4;
   const int64_t total = static_cast<int64_t>(M) * n4;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;

@@ -131,6 +131,14 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
+// ---- dependent launches ------------------------------------------------------------------
+// A kernel launched with `dependent_launch` may start while the kernel before it in the stream still runs, once every block of that one
+// has called `let_dependents_start` or ended: its set-up (barriers, tensor memory, descriptors) then lies behind the other's tail.
+// `wait_for_stream` returns when everything before is complete and visible. Every thread of such a kernel calls it before it touches
+// global memory; the kernel before needs no such care, whatever it is.
+__device__ __forceinline__ void wait_for_stream() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_dependents_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- TMA (tiled bulk tensor copies; never multicast) -----------------------------------
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* m) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(m)) : "memory");

@@ -61,6 +61,7 @@ template <int NV, int WPR, int MODE>
 __global__ void norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gamma,
                                 const __nv_bfloat16* __restrict__ beta, __nv_bfloat16* __restrict__ y,
                                 float* __restrict__ mean_out, float* __restrict__ rstd_out, int M, int D, float eps) {
+  let_dependents_start();
   constexpr int ROWS = 4 / WPR > 0 ? 4 / WPR : 1;  // rows per block (128 or 32*WPR threads)
   __shared__ float scratch[ROWS * WPR + 1];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -136,6 +137,7 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __res
                                 const __nv_bfloat16* __restrict__ gamma, const float* __restrict__ mean_in,
                                 const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ dres,
                                 __nv_bfloat16* __restrict__ dx, float* __restrict__ partials, int M, int D) {
+  let_dependents_start();
   constexpr int ROWS = 4 / WPR > 0 ? 4 / WPR : 1;
   __shared__ float scratch[ROWS * WPR + 1];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -224,6 +226,7 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __res
 constexpr int kNormReduceSlices = 8;
 __global__ void norm_bwd_reduce_kernel(const float* __restrict__ partials, int n_rows, int D, int with_beta,
                                        float* __restrict__ dgamma, float* __restrict__ dbeta) {
+  let_dependents_start();
   __shared__ float red[32][33];
   const int width = with_beta ? 2 * D : D;
   const int c = blockIdx.x * 32 + threadIdx.x;  // column in the concatenated [dgamma | dbeta] row
@@ -344,6 +347,7 @@ __global__ void embed_bwd_kernel(const int32_t* __restrict__ idx, const __nv_bfl
 __global__ void __launch_bounds__(512)
 ce_fwd_bwd_kernel(__nv_bfloat16* __restrict__ logits, const int32_t* __restrict__ targets,
                   float* __restrict__ loss, int V, int ldl, float scale, int write_grad) {
+  let_dependents_start();
   __shared__ float red[32];
   __shared__ float bcast[2];
   const int row = blockIdx.x;
@@ -410,6 +414,7 @@ ce_fwd_bwd_kernel(__nv_bfloat16* __restrict__ logits, const int32_t* __restrict_
 // dbias[c] += sum_rows dy[r, c]. Block = 32 x 8 threads handling a 256-column strip.
 __global__ void bias_grad_kernel(const __nv_bfloat16* __restrict__ dy, float* __restrict__ dbias, int M, int N,
                                  int rows_per_block) {
+  let_dependents_start();
   __shared__ float acc[8][256 + 8];
   const int tx = threadIdx.x, ty = threadIdx.y;
   const int col = blockIdx.x * 256 + tx * 8;

@@ -158,6 +158,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
   cluster_sync_all();  // the peer's barriers are initialised before anything signals them
   tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
+  let_dependents_start();
+  wait_for_stream();
 
   // Linear pair-tile index -> (256-row block, 256-column block, k split); bands of kBand row blocks
   // keep the tiles that run together inside a small set of A and B panels (L2 reuse).
@@ -328,8 +330,15 @@ cudaError_t launch_pair_variant(const CUtensorMap& ta, const CUtensorMap& tb, co
   }
   const int max_pairs = gemm_sm_count() / 2;
   const int pairs = tiles < max_pairs ? tiles : max_pairs;
-  kernel<<<2 * pairs, kNumThreads, kSmemBytes, stream>>>(ta, tb, args);
-  return cudaGetLastError();
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(2 * pairs);
+  cfg.blockDim = dim3(kNumThreads);
+  cfg.dynamicSmemBytes = kSmemBytes;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr = dependent_launch();
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, ta, tb, args);
 }
 
 }  // namespace

@@ -250,6 +250,8 @@ gemm_bf16_kernel(const __grid_constant__ TmaSet tma_a, const __grid_constant__ T
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
+  let_dependents_start();
+  wait_for_stream();
 
   // Maps a linear tile index to (m block, n block, k split). Consecutive tiles share the
   // B tile so the CTAs running together re-use it out of L2. With gathered A the m blocks
@@ -566,28 +568,24 @@ cudaError_t launch_variant(const TmaSet& ta, const TmaSet& tb, const GemmArgs& a
   }
   const int m_blocks = (args.M + BM - 1) / BM;
   const int n_blocks = (args.N + BN - 1) / BN;
-  if (args.cluster_k > 1) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(m_blocks * n_blocks * args.cluster_k);
-    cfg.blockDim = dim3(kNumThreads);
-    cfg.dynamicSmemBytes = C::kSmemBytes;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = args.cluster_k;
-    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, ta, tb, args, gi, sc);
-  }
   const int tiles = m_blocks * n_blocks * (args.split_k < 1 ? 1 : args.split_k);
   // copier CTAs must be resident together with the compute CTAs that wait for them: the grid never exceeds the
   // SM count (one CTA per SM by shared memory)
   const int room = gemm_sm_count() - sc.n_copy_ctas;
   if (room < 1) return cudaErrorInvalidValue;
   const int grid = (tiles < room ? tiles : room) + sc.n_copy_ctas;
-  kernel<<<grid, kNumThreads, C::kSmemBytes, stream>>>(ta, tb, args, gi, sc);
-  return cudaGetLastError();
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(args.cluster_k > 1 ? m_blocks * n_blocks * args.cluster_k : grid);
+  cfg.blockDim = dim3(kNumThreads);
+  cfg.dynamicSmemBytes = C::kSmemBytes;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2] = {dependent_launch(), {}};
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = args.cluster_k;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = sc.n_copy_ctas > 0 ? 0 : (args.cluster_k > 1 ? 2 : 1);   // copiers start with their peers' kernels, not early
+  return cudaLaunchKernelEx(&cfg, kernel, ta, tb, args, gi, sc);
 }
 
 cudaError_t make_operand_map(CUtensorMap* map, const __nv_bfloat16* p, int64_t ld, int major, int rows_mn, int K,

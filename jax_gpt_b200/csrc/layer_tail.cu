@@ -42,6 +42,7 @@ __device__ __forceinline__ void unpack8(uint4 u, float (&f)[8]) {
 // by latency for few.
 template <int NV>
 __global__ void __launch_bounds__(256) layer_tail_kernel(const LayerTailArgs a) {
+  let_dependents_start();
   __shared__ float scratch[8];
   const int64_t row = blockIdx.x, base = row * a.D;
   const int n8 = a.D / 8;
@@ -148,6 +149,7 @@ moe_prepare_zero_kernel(const int* __restrict__ idx, int n_pairs, int n_experts,
 __global__ void __launch_bounds__(256)
 silu_mul_kernel(const __nv_bfloat16* __restrict__ g, int64_t ldg, const __nv_bfloat16* __restrict__ u, int64_t ldu,
                 __nv_bfloat16* __restrict__ out, int64_t n8, int i8) {
+  let_dependents_start();
   const int64_t step = static_cast<int64_t>(gridDim.x) * blockDim.x;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n8; i += step) {
     const int64_t row = i / i8, c = i - row * i8;

@@ -45,6 +45,7 @@ __device__ __forceinline__ void warp_argmax(float& v, int& i) {
 __global__ void router_kernel(int mode, const float* __restrict__ logits, const float* __restrict__ bias, int M, int E,
                               int k, int n_group, int topk_group, float scale, float* __restrict__ weights,
                               int* __restrict__ ids, int* __restrict__ counts) {
+  let_dependents_start();
   const int tok = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (tok >= M) return;
@@ -516,6 +517,7 @@ mla_step_rope_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* _
                      const __nv_bfloat16* __restrict__ kv, const __nv_bfloat16* __restrict__ c_kv, const float* __restrict__ freqs,
                      const int64_t* __restrict__ pos, __nv_bfloat16* __restrict__ q_full, __nv_bfloat16* __restrict__ lat, int H, int dn,
                      int dr, int kvr) {
+  let_dependents_start();
   const int64_t b = blockIdx.x;
   const int half = dr / 2, dq = dn + dr, W = kvr + dr, h0 = blockIdx.y * 8;
   const float2* fr = reinterpret_cast<const float2*>(freqs) + pos[b] * half;
@@ -576,6 +578,7 @@ gdn_decode_128_kernel(const __nv_bfloat16* __restrict__ mixed, const __nv_bfloat
                       const __nv_bfloat16* __restrict__ dt_bias, const __nv_bfloat16* __restrict__ norm_w,
                       float* __restrict__ state, __nv_bfloat16* __restrict__ out, int Hqk, int Hv, float eps, int ld_mixed, int ld_z,
                       int ld_b, int ld_a) {
+  let_dependents_start();
   constexpr int D = kGdnDim, kWarps = 8, kRows = D / kWarps;
   __shared__ float qk[2][D], vs[D], scratch[kWarps];
   __shared__ float4 red[kWarps][D / 4];

@@ -7,6 +7,14 @@
 
 namespace b200 {
 
+// Launch attribute of a kernel that calls wait_for_stream (common.cuh) before it touches global memory.
+inline cudaLaunchAttribute dependent_launch() {
+  cudaLaunchAttribute a{};
+  a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  a.val.programmaticStreamSerializationAllowed = 1;
+  return a;
+}
+
 // 2-D tiled map with 128-byte swizzle. `inner` / `outer` are extents in elements, the row
 // stride is in bytes (multiple of 16), the box is `box_inner` x `box_outer` elements and
 // box_inner * elem_bytes must equal 128.
