@@ -158,3 +158,19 @@ def test_decode_of_shared_kv_heads(cuda_device, D, Dv, H, Hkv, window, keep, cap
         ref = torch.einsum("hn,nhd->hd", torch.softmax(sc, -1)[:, :n], v)
         rel = ((out[b].float() - ref).norm() / ref.norm()).item()
         assert rel < 4e-3, (n, rel)
+
+
+@pytest.mark.parametrize("B,T,H,Hkv,causal", [(1, 130, 8, 1, True), (2, 64, 4, 2, True), (1, 300, 6, 1, False), (1, 129, 2, 1, True), (3, 700, 8, 2, True)])
+def test_wide_backward_shares_query_heads(cuda_device, B, T, H, Hkv, causal):
+    """Width 256 with eight, six (no power of two: clusters of two), four and two query heads per kv head: the clusters' partial dK and dV
+    add up. P, dS and the outputs are rounded to bf16, a few times 2^-9 each."""
+    from jax_gpt_b200.ops.attention import attention, attention_ref
+    g = torch.Generator(device=cuda_device).manual_seed(31)
+    rnd = lambda *s: torch.randn(*s, device=cuda_device, generator=g).to(torch.bfloat16)
+    q, k, v, do = rnd(B, T, H, 256), rnd(B, T, Hkv, 256), rnd(B, T, Hkv, 256), rnd(B, T, H, 256)
+    ins = [t.requires_grad_(True) for t in (q, k, v)]
+    got = torch.autograd.grad(attention(*ins, causal=causal), ins, do)
+    f32 = [t.detach().float().requires_grad_(True) for t in ins]
+    want = torch.autograd.grad(attention_ref(*f32, causal=causal), f32, do.float())
+    for a, b in zip(got, want):
+        assert _rel_err(a, b) < 1.5e-2, _rel_err(a, b)
