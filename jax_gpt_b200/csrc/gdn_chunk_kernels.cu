@@ -1,5 +1,5 @@
 // Gated-DeltaNet prefill: everything of the chunked gated delta rule that does NOT depend on the running state,
-// forward and backward, as one kernel each (fp32 on the CUDA cores, no library call).
+// forward and backward, as one kernel each (matrix instructions around an fp32 inverse, no library call).
 //
 // Per chunk of 64 tokens and per value head the chunked algorithm needs (jax_gpt/models/qwen35/deltanet.py:214-300,
 // which computes them with batched einsums and a triangular solve):
@@ -10,18 +10,12 @@
 //     intra = lower(q^_i . k^_j exp(G_i - G_j))               k_dec = k^ exp(G_end - G)      q_e = q^ exp(G)
 // and the inter-chunk scan (gdn_kernels.cu) consumes [k_cum ; q_e], intra, k_dec, v_eff, exp(G_end).
 //
-// One CTA of 256 threads owns one (batch, q/k head, chunk) and loops over the value heads that share the q/k head:
-// the normalised q and k tiles stay in shared memory as fp32, the 64 x 64 Gram matrices are computed by a 16 x 16
-// thread grid (4 x 4 interleaved entries each), and the unit-lower-triangular solve is a forward substitution with
-// one right-hand-side COLUMN per thread held in 64 registers (256 columns = 256 threads), so it needs no barriers.
+// One CTA owns one (batch, q/k head, chunk) and loops over the value heads that share the q/k head. The raw bf16 rows of q, k and
+// v lie in shared memory as they are; every product with them is exact in its operands, their L2 norms scale fp32 sums or factors.
 //
-// The backward kernel recomputes the forward quantities from the same inputs, solves the transposed system
-// Y = (I + A)^-T dX by backward substitution (again one column per thread), forms dA = -strict_lower(Y X^T), and
-// pushes the gradients through the decays, the gates, the Gram matrices and the two L2 norms down to d(mixed),
-// d(b), d(a), d(A_log) and d(dt_bias). Gradients of q and k are summed over the value heads on chip, so the kernel
-// has no global atomics except the two per-head scalars. Those 2 x 64 x 128 fp32 sums are thread-private (64 values
-// per thread) but must survive the substitution phases, which need every register for the 64-entry columns; shared
-// memory is full, so they are parked in tensor memory (tcgen05.st / tcgen05.ld, 128 columns) between the phases.
+// The backward kernel recomputes the forward quantities from the same inputs and pushes the gradients through the solve, the
+// decays, the gates, the Gram matrices and the two L2 norms down to d(mixed), d(b), d(a), d(A_log) and d(dt_bias). Gradients of q
+// and k are summed over the value heads in registers, so the kernel has no global atomics except the two per-head scalars.
 #include "seq_kernels.cuh"
 
 #include "common.cuh"
@@ -32,7 +26,6 @@ namespace {
 
 constexpr int kC = 64;            // chunk length
 constexpr int kD = 128;           // dk = dv
-constexpr int kLd = kD + 4;       // row stride (floats) of the 64 x 128 fp32 tiles in shared memory
 constexpr int kThreads = 256;
 constexpr float kQScale = 0.08838834764831845f;   // 128^-1/2
 
@@ -46,127 +39,6 @@ __device__ __forceinline__ float bf2f(const __nv_bfloat16* p) { return __bfloat1
 __device__ __forceinline__ float2 bf2f2(const __nv_bfloat16* p) {
   return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p));
 }
-__device__ __forceinline__ float dot4(const float4& a, const float4& b) { return a.x * b.x + a.y * b.y + a.z * b.z + a.w * b.w; }
-
-// Loads the chunk's q and k rows (bf16, 128 wide each) as fp32 into sq / sk, L2-normalises every row (q is also
-// scaled by dk^-1/2) and leaves the reciprocal norms in s_rq / s_rk. Rows at or beyond T become zero.
-__device__ void load_qk_normalised(const __nv_bfloat16* mixed_b, const PrepGeom& gm, int n, int hq, float* sq, float* sk,
-                                   float* s_rq, float* s_rk) {
-  const int tid = threadIdx.x;
-  for (int idx = tid; idx < 2 * kC * 16; idx += kThreads) {
-    const int which = idx / (kC * 16), rem = idx % (kC * 16);
-    const int i = rem / 16, v8 = rem % 16;
-    const int t = n * kC + i;
-    float* dst = (which ? sk : sq) + i * kLd + v8 * 8;
-    if (t < gm.T) {
-      const uint4 raw = *reinterpret_cast<const uint4*>(mixed_b + static_cast<size_t>(t) * gm.conv_dim +
-                                                        which * gm.Hqk * kD + hq * kD + v8 * 8);
-      const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&raw);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float2 f = __bfloat1622float2(p[e]);
-        dst[2 * e] = f.x;
-        dst[2 * e + 1] = f.y;
-      }
-    } else {
-#pragma unroll
-      for (int e = 0; e < 8; ++e) dst[e] = 0.f;
-    }
-  }
-  __syncthreads();
-  const int i = tid >> 2, qd = tid & 3;
-  float ssq = 0.f, ssk = 0.f;
-#pragma unroll
-  for (int m = 0; m < 16; ++m) {
-    const float2 a = *reinterpret_cast<const float2*>(sq + i * kLd + 2 * (qd + 4 * m));
-    const float2 b = *reinterpret_cast<const float2*>(sk + i * kLd + 2 * (qd + 4 * m));
-    ssq += a.x * a.x + a.y * a.y;
-    ssk += b.x * b.x + b.y * b.y;
-  }
-  ssq += __shfl_xor_sync(0xffffffffu, ssq, 1);
-  ssq += __shfl_xor_sync(0xffffffffu, ssq, 2);
-  ssk += __shfl_xor_sync(0xffffffffu, ssk, 1);
-  ssk += __shfl_xor_sync(0xffffffffu, ssk, 2);
-  const float rq = rsqrtf(ssq + 1e-6f), rk = rsqrtf(ssk + 1e-6f);
-#pragma unroll
-  for (int m = 0; m < 16; ++m) {
-    float2* a = reinterpret_cast<float2*>(sq + i * kLd + 2 * (qd + 4 * m));
-    float2* b = reinterpret_cast<float2*>(sk + i * kLd + 2 * (qd + 4 * m));
-    a->x *= rq * kQScale;
-    a->y *= rq * kQScale;
-    b->x *= rk;
-    b->y *= rk;
-  }
-  if (qd == 0) {
-    s_rq[i] = rq;
-    s_rk[i] = rk;
-  }
-  __syncthreads();
-}
-
-// Thread (ti, tj) of the 16 x 16 grid owns entries (ti + 16 a, tj + 16 b): s = k^ k^T, w = q^ k^T. Entries above
-// the diagonal are never used, so block columns b > a are skipped.
-__device__ __forceinline__ void gram_blocks(const float* sq, const float* sk, int ti, int tj, float (&s)[4][4],
-                                            float (&w)[4][4]) {
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int b = 0; b < 4; ++b) s[a][b] = w[a][b] = 0.f;
-#pragma unroll 2
-  for (int c = 0; c < kD; c += 4) {
-    float4 ki[4], qi[4], kj[4];
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-      ki[a] = *reinterpret_cast<const float4*>(sk + (ti + 16 * a) * kLd + c);
-      qi[a] = *reinterpret_cast<const float4*>(sq + (ti + 16 * a) * kLd + c);
-      kj[a] = *reinterpret_cast<const float4*>(sk + (tj + 16 * a) * kLd + c);
-    }
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int b = 0; b < 4; ++b)
-        if (b <= a) {
-          s[a][b] += dot4(ki[a], kj[b]);
-          w[a][b] += dot4(qi[a], kj[b]);
-        }
-  }
-}
-
-// Gates of one value head for the 64 rows of the chunk (threads 0..63 compute, everybody leaves synchronised):
-// s_beta, s_g (raw log-decay), s_G (inclusive cumulative sum), s_eg = exp(G), s_ed = exp(G_end - G), s_asig =
-// sigmoid(a + dt_bias) (the derivative of the softplus). Rows at or beyond T have beta = g = 0.
-__device__ void chunk_gates(const __nv_bfloat16* b_in, const __nv_bfloat16* a_in, float a_neg, float dtb,
-                            const PrepGeom& gm, int batch, int n, int hv, float* s_beta, float* s_g, float* s_G,
-                            float* s_eg, float* s_ed, float* s_asig) {
-  const int tid = threadIdx.x;
-  if (tid < kC) {
-    const int t = n * kC + tid;
-    float beta = 0.f, g = 0.f, asig = 0.f;
-    if (t < gm.T) {
-      const size_t off = (static_cast<size_t>(batch) * gm.T + t) * gm.Hv + hv;
-      beta = sigmoid_f(bf2f(b_in + off));
-      const float x = bf2f(a_in + off) + dtb;
-      g = a_neg * softplus_f(x);
-      asig = sigmoid_f(x);
-    }
-    s_beta[tid] = beta;
-    s_g[tid] = g;
-    s_asig[tid] = asig;
-  }
-  __syncthreads();
-  if (tid < kC) {
-    float G = 0.f;
-    for (int j = 0; j <= tid; ++j) G += s_g[j];
-    s_G[tid] = G;
-  }
-  __syncthreads();
-  if (tid < kC) {
-    s_eg[tid] = expf(s_G[tid]);
-    s_ed[tid] = expf(s_G[kC - 1] - s_G[tid]);
-  }
-  __syncthreads();
-}
-
 struct PrepFwdArgs {
   const __nv_bfloat16* mixed;   // [B, T, conv_dim]: q | k | v after conv + SiLU
   const __nv_bfloat16* b_in;    // [B, T, Hv]
@@ -218,9 +90,10 @@ __device__ __forceinline__ void ldsm4_t(uint32_t (&r)[4], const void* p) {
 }
 
 // 64 rows of 128 features from column `col` of the projections, zeros from row T on.
+template <int NT>
 __device__ __forceinline__ void load_raw_tile(const __nv_bfloat16* mixed_b, const PrepGeom& gm, int n, int col, __nv_bfloat16* dst) {
 #pragma unroll
-  for (int i = threadIdx.x; i < kC * (kD / 8); i += kThreads) {
+  for (int i = threadIdx.x; i < kC * (kD / 8); i += NT) {
     const int r = i >> 4, c8 = i & 15, t = n * kC + r;
     uint4 u = make_uint4(0, 0, 0, 0);
     if (t < gm.T) u = *reinterpret_cast<const uint4*>(mixed_b + static_cast<size_t>(t) * gm.conv_dim + col + c8 * 8);
@@ -230,11 +103,11 @@ __device__ __forceinline__ void load_raw_tile(const __nv_bfloat16* mixed_b, cons
 
 // out (rows x cols) = sign * a (rows x inner) b (inner x cols), fp32 in shared memory, a thread per output, rows * cols a multiple
 // of the block; `blocks` such products, the operands a step apart.
-template <int kRows, int kCols, int kInner>
+template <int NT, int kRows, int kCols, int kInner>
 __device__ __forceinline__ void small_product(float* out, int ldo, const float* a, int lda, const float* b, int ldb, float sign,
                                               int blocks, int out_step, int a_step, int b_step) {
   const int per = kRows * kCols;
-  for (int o = threadIdx.x; o < blocks * per; o += kThreads) {
+  for (int o = threadIdx.x; o < blocks * per; o += NT) {
     const int blk = o / per, r = (o % per) / kCols, c = o % kCols;
     const float* ar = a + blk * a_step + r * lda;
     const float* bc = b + blk * b_step + c;
@@ -252,6 +125,7 @@ __device__ __forceinline__ void small_product(float* out, int ldo, const float* 
 }
 
 // T = (I + A)^-1 of the strictly lower triangular A; blocks of T above the diagonal that a product reads are cleared.
+template <int NT>
 __device__ __forceinline__ void unit_lower_inverse(const float* A, float* T, float* U) {
   const int tid = threadIdx.x;
   if (tid < kC) {
@@ -266,19 +140,19 @@ __device__ __forceinline__ void unit_lower_inverse(const float* A, float* T, flo
       T[(b0 + i) * kTLd + tid] = x[i];
     }
   } else if (tid >= 128) {
-    for (int i = tid - 128; i < 512; i += 128) {   // the blocks right of the first and of the third on the diagonal
+    for (int i = tid - 128; i < 512; i += NT - 128) {   // the blocks right of the first and of the third on the diagonal
       const int r = (i >> 8) * 32 + ((i >> 4) & 15), c = (i >> 8) * 32 + 16 + (i & 15);
       T[r * kTLd + c] = 0.f;
     }
   }
   __syncthreads();
-  small_product<16, 16, 16>(U, kULd, A + 16 * kALd, kALd, T, kTLd, 1.f, 2, 16 * kULd, 32 * kALd + 32, 32 * kTLd + 32);
+  small_product<NT, 16, 16, 16>(U, kULd, A + 16 * kALd, kALd, T, kTLd, 1.f, 2, 16 * kULd, 32 * kALd + 32, 32 * kTLd + 32);
   __syncthreads();
-  small_product<16, 16, 16>(T + 16 * kTLd, kTLd, T + 16 * kTLd + 16, kTLd, U, kULd, -1.f, 2, 32 * kTLd + 32, 32 * kTLd + 32, 16 * kULd);
+  small_product<NT, 16, 16, 16>(T + 16 * kTLd, kTLd, T + 16 * kTLd + 16, kTLd, U, kULd, -1.f, 2, 32 * kTLd + 32, 32 * kTLd + 32, 16 * kULd);
   __syncthreads();
-  small_product<32, 32, 32>(U, kULd, A + 32 * kALd, kALd, T, kTLd, 1.f, 1, 0, 0, 0);
+  small_product<NT, 32, 32, 32>(U, kULd, A + 32 * kALd, kALd, T, kTLd, 1.f, 1, 0, 0, 0);
   __syncthreads();
-  small_product<32, 32, 32>(T + 32 * kTLd, kTLd, T + 32 * kTLd + 32, kTLd, U, kULd, -1.f, 1, 0, 0, 0);
+  small_product<NT, 32, 32, 32>(T + 32 * kTLd, kTLd, T + 32 * kTLd + 32, kTLd, U, kULd, -1.f, 1, 0, 0, 0);
   __syncthreads();
 }
 
@@ -290,8 +164,8 @@ __global__ void __launch_bounds__(kThreads, 2) gdn_chunk_prep_fwd_kernel(const P
   const int n = blockIdx.x, hq = blockIdx.y, batch = blockIdx.z;
   const int rep = gm.Hv / gm.Hqk;
   const __nv_bfloat16* mixed_b = p.mixed + static_cast<size_t>(batch) * gm.T * gm.conv_dim;
-  load_raw_tile(mixed_b, gm, n, hq * kD, sm.q);
-  load_raw_tile(mixed_b, gm, n, gm.Hqk * kD + hq * kD, sm.k);
+  load_raw_tile<kThreads>(mixed_b, gm, n, hq * kD, sm.q);
+  load_raw_tile<kThreads>(mixed_b, gm, n, gm.Hqk * kD + hq * kD, sm.k);
   __syncthreads();
   {
     // reciprocal norms, four threads per row
@@ -355,8 +229,8 @@ __global__ void __launch_bounds__(kThreads, 2) gdn_chunk_prep_fwd_kernel(const P
   for (int r = 0; r < rep; ++r) {
     const int hv = hq * rep + r;
     const size_t chunk = (static_cast<size_t>(batch) * gm.Hv + hv) * gm.N + n;
-    load_raw_tile(mixed_b, gm, n, 2 * gm.Hqk * kD + hv * kD, sm.v);
-    // gates (see chunk_gates), the cumulative sum by two warps
+    load_raw_tile<kThreads>(mixed_b, gm, n, 2 * gm.Hqk * kD + hv * kD, sm.v);
+    // gates, the cumulative sum by two warps; rows at or beyond T have beta = g = 0
     float beta = 0.f, G = 0.f;
     if (tid < kC) {
       const int t = n * kC + tid;
@@ -404,7 +278,7 @@ __global__ void __launch_bounds__(kThreads, 2) gdn_chunk_prep_fwd_kernel(const P
       }
     }
     __syncthreads();
-    unit_lower_inverse(sm.A, sm.T, sm.U);
+    unit_lower_inverse<kThreads>(sm.A, sm.T, sm.U);
     {
       // X = (T diag(s)) R: warps 0-3 the value columns (s = beta), warps 4-7 the key columns (s = beta exp(G) / |k|), 32 columns each
       const __nv_bfloat16* right = (of_q ? sm.k : sm.v) + mt * 32;
@@ -492,360 +366,483 @@ struct PrepBwdArgs {
   PrepGeom gm;
 };
 
-constexpr int kBwdSmemFloats = 4 * kC * kLd + 3 * kC * kC + 10 * kC + 4;
+// ---- backward ----------------------------------------------------------------------------------------------------------
+// With T = (I + A)^-1, X = T R and the incoming dX: Y = T^T dX is the gradient of the right-hand sides R, and that of A is
+// -strict_lower(Y X^T) = -strict_lower(T^T (dX R^T) T^T), so X itself is not needed. dX and the raw rows of R are bf16, products with
+// them are matrix instructions with an fp32 factor in three bf16 parts as in the forward kernel; the two 64 x 64 x 64 products with T
+// on both sides are fp32. One CTA of 16 warps: the 64 x 128 sums of dQ and dK over the value heads stay in registers (warps 0-7 dQ, 8-15
+// dK, a row tile and 64 columns each).
+//
+// The kernel before solved the two triangular systems with a column of 64 registers per thread and formed Y X^T and three products with
+// dS, dW, dW^T on the CUDA cores, 800 us for 2048 tokens and 32 value heads; here 249 us. The terms
+// of dG (the gates' cumulative sums) largely cancel: they are added up in 64 bits, which halves to quarters the error of d(A_log), d(dt_bias).
+constexpr int kBwdThreads = 512;
 
-__global__ void __launch_bounds__(kThreads, 1) gdn_chunk_prep_bwd_kernel(const PrepBwdArgs p) {
-  extern __shared__ __align__(16) float smem[];
-  float* sq = smem;
-  float* sk = sq + kC * kLd;
-  float* sX = sk + kC * kLd;
-  float* sY = sX + kC * kLd;
-  float* sM0 = sY + kC * kLd;        // k^ k^T * decay (strict lower), later dS + dS^T
-  float* sM1 = sM0 + kC * kC;        // q^ k^T * decay (lower), later dW
-  float* sM2 = sM1 + kC * kC;        // dW^T
-  float* s_beta = sM2 + kC * kC;
-  float* s_g = s_beta + kC;
-  float* s_G = s_g + kC;
-  float* s_eg = s_G + kC;
-  float* s_ed = s_eg + kC;
-  float* s_asig = s_ed + kC;
-  float* s_rq = s_asig + kC;
-  float* s_rk = s_rq + kC;
-  float* s_dG = s_rk + kC;
-  float* s_dbeta = s_dG + kC;
-  uint32_t* s_tmem = reinterpret_cast<uint32_t*>(s_dbeta + kC);
+struct PrepBwdSmem {
+  __nv_bfloat16 q[kC * kRawLd], k[kC * kRawLd], v[kC * kRawLd], dxv[kC * kRawLd], dxk[kC * kRawLd];
+  float A[kC * kALd], M0[kC * kALd], N[kC * kALd];     // M0: k^ k^T with the decays, strictly lower; A = beta M0; N = dX R^T
+  float T[kC * kTLd], P[kC * kTLd], S[kC * kTLd], W[kC * kTLd], U[32 * kULd];   // P = N T^T; S = dS + dS^T; W = dW
+  float beta[kC], g[kC], G[kC], eg[kC], ed[kC], asig[kC], rq[kC], rk[kC], kscale[kC];
+  double dG[kC];                     // its terms largely cancel in the sums from a row to the end
+  float dbeta[kC], dotq[kC], dotk[kC];
+  float warp0_sum;
+};
+static_assert(sizeof(PrepBwdSmem) <= 227 * 1024, "shared memory");
+
+__device__ __forceinline__ void load_chunk_tile(const __nv_bfloat16* src, __nv_bfloat16* dst) {   // 64 x 128, contiguous
+  for (int i = threadIdx.x; i < kC * (kD / 8); i += kBwdThreads)
+    *reinterpret_cast<uint4*>(dst + (i >> 4) * kRawLd + (i & 15) * 8) = reinterpret_cast<const uint4*>(src)[i];
+}
+template <class F>
+__device__ __forceinline__ F quad_sum(F v) {     // over the four lanes that share a fragment's row
+  v += __shfl_xor_sync(0xffffffffu, v, 1);
+  return v + __shfl_xor_sync(0xffffffffu, v, 2);
+}
+__device__ __forceinline__ double column_sum(double v) {   // over the eight lanes that share a fragment's column
+  v += __shfl_xor_sync(0xffffffffu, v, 4);
+  v += __shfl_xor_sync(0xffffffffu, v, 8);
+  return v + __shfl_xor_sync(0xffffffffu, v, 16);
+}
+
+// The matrix unit cuts its sums off instead of rounding them: every step of 16 starts at zero and is added on with rounding.
+__device__ __forceinline__ void add4(float (&acc)[4], const float (&x)[4]) {
+#pragma unroll
+  for (int e = 0; e < 4; ++e) acc[e] += x[e];
+}
+__device__ __forceinline__ void mma_add(float (&acc)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  float x[4] = {};
+  mma_16816(x, a, b0, b1);
+  add4(acc, x);
+}
+
+// acc (16 rows x 8 * NT columns of fragments) += left (16 x 16 per step, fp32 by `load(row, col)` = columns col, col + 1) right, over
+// the steps [k0, k1) of 16; `right` points at the first of the columns in a raw tile.
+template <int NT, class Load>
+__device__ __forceinline__ void split_product(float (&acc)[NT][4], const Load& load, int k0, int k1, const __nv_bfloat16* right) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
+#pragma unroll 1
+  for (int ks = k0; ks < k1; ++ks) {
+    uint32_t part[3][4];
+#pragma unroll
+    for (int f = 0; f < 4; ++f) {
+      float2 x = load(g + (f & 1) * 8, ks * 16 + 2 * t4 + (f >> 1) * 8);
+#pragma unroll
+      for (int e = 0; e < 3; ++e) {
+        part[e][f] = pack_bf16x2(x.x, x.y);
+        const float2 h = unpack_bf16x2(part[e][f]);
+        x.x -= h.x;
+        x.y -= h.y;
+      }
+    }
+#pragma unroll
+    for (int j2 = 0; j2 < NT / 2; ++j2) {
+      uint32_t b[4];
+      ldsm4_t(b, right + (ks * 16 + ((lane >> 3) & 1) * 8 + (lane & 7)) * kRawLd + j2 * 16 + (lane >> 4) * 8);
+      float lo[4] = {}, hi[4] = {};
+#pragma unroll
+      for (int e = 2; e >= 0; --e) {  // the small parts first
+        mma_16816(lo, part[e], b[0], b[1]);
+        mma_16816(hi, part[e], b[2], b[3]);
+      }
+      add4(acc[2 * j2], lo);
+      add4(acc[2 * j2 + 1], hi);
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kBwdThreads, 1) gdn_chunk_prep_bwd_kernel(const PrepBwdArgs p) {
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  PrepBwdSmem& sm = *reinterpret_cast<PrepBwdSmem*>(smem_raw);
   const PrepGeom gm = p.gm;
-  const int tid = threadIdx.x, n = blockIdx.x, hq = blockIdx.y, batch = blockIdx.z;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
+  const int n = blockIdx.x, hq = blockIdx.y, batch = blockIdx.z;
   const int rep = gm.Hv / gm.Hqk;
   const size_t tok0 = static_cast<size_t>(batch) * gm.T;
   const __nv_bfloat16* mixed_b = p.mixed + tok0 * gm.conv_dim;
   __nv_bfloat16* d_mixed_b = p.d_mixed + tok0 * gm.conv_dim;
-  load_qk_normalised(mixed_b, gm, n, hq, sq, sk, s_rq, s_rk);
-  const int ti = tid >> 4, tj = tid & 15;     // Gram-matrix mapping
-  const int ri = tid >> 2, rqd = tid & 3;     // row mapping: row ri, column pairs rqd + 4 m
-  const int cc = tid & 127, hb = tid >> 7;    // column mapping: column cc, rows 2 m + hb
-  // gradients of the scaled q^ and of k^, summed over the value heads: parked in tensor memory, this thread's lane
-  // (warp % 4 selects the lane quadrant) and 64 columns (dq: 0-31, dk: 32-63 of the warp's column group)
-  if (tid < 32) {
-    tmem_alloc(s_tmem, 128);
-    tmem_relinquish();
-  }
-  tc_fence_before();
+  load_raw_tile<kBwdThreads>(mixed_b, gm, n, hq * kD, sm.q);
+  load_raw_tile<kBwdThreads>(mixed_b, gm, n, gm.Hqk * kD + hq * kD, sm.k);
   __syncthreads();
-  tc_fence_after();
-  const uint32_t park = *s_tmem + ((static_cast<uint32_t>((tid >> 5) & 3) * 32u) << 16) + static_cast<uint32_t>(tid >> 7) * 64u;
   {
-    uint32_t z[32];
+    // reciprocal norms, eight threads per row
+    const int i = tid >> 3, qd = tid & 7;
+    float ssq = 0.f, ssk = 0.f;
 #pragma unroll
-    for (int m = 0; m < 32; ++m) z[m] = 0u;
-    tmem_st_32x32(park, z);
-    tmem_st_32x32(park + 32, z);
-    tmem_st_wait();
+    for (int m = 0; m < 2; ++m) {
+      const uint4 a = *reinterpret_cast<const uint4*>(sm.q + i * kRawLd + (qd + 8 * m) * 8);
+      const uint4 b = *reinterpret_cast<const uint4*>(sm.k + i * kRawLd + (qd + 8 * m) * 8);
+      const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, bw[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 x = unpack_bf16x2(aw[e]), y = unpack_bf16x2(bw[e]);
+        ssq += x.x * x.x + x.y * x.y;
+        ssk += y.x * y.x + y.y * y.y;
+      }
+    }
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) {
+      ssq += __shfl_xor_sync(0xffffffffu, ssq, o);
+      ssk += __shfl_xor_sync(0xffffffffu, ssk, o);
+    }
+    if (qd == 0) {
+      sm.rq[i] = rsqrtf(ssq + 1e-6f) * kQScale;
+      sm.rk[i] = rsqrtf(ssk + 1e-6f);
+    }
   }
+  for (int i = tid; i < kC; i += kBwdThreads) sm.dotq[i] = sm.dotk[i] = 0.f;
+  __syncthreads();
+  const int mt = warp & 3, row_lo = mt * 16 + g, row_hi = row_lo + 8, part = (warp >> 2) & 1;
+  const bool second = warp >= 8;     // Gram matrix of q^, key columns, dK; the first eight warps: of k^, value columns, dQ
+  // Gram matrices (32 columns per warp, nothing above the diagonal)
+  float gram[4][4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) gram[j][0] = gram[j][1] = gram[j][2] = gram[j][3] = 0.f;
+  {
+    const __nv_bfloat16* left = second ? sm.q : sm.k;
+#pragma unroll
+    for (int ks = 0; ks < kD / 16; ++ks) {
+      uint32_t a[4];
+      ldsm4(a, left + (mt * 16 + (lane & 15)) * kRawLd + ks * 16 + (lane >> 4) * 8);
+#pragma unroll
+      for (int jj = 0; jj < 2; ++jj) {
+        const int cb = part * 2 + jj;
+        if (cb > mt) continue;
+        uint32_t b[4];
+        ldsm4(b, sm.k + (cb * 16 + (lane >> 4) * 8 + (lane & 7)) * kRawLd + ks * 16 + ((lane >> 3) & 1) * 8);
+        mma_add(gram[2 * jj], a, b[0], b[1]);
+        mma_add(gram[2 * jj + 1], a, b[2], b[3]);
+      }
+    }
+    const float* rl = second ? sm.rq : sm.rk;
+    const float lo = rl[row_lo], hi = rl[row_hi];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float c0 = sm.rk[part * 32 + j * 8 + 2 * t4], c1 = sm.rk[part * 32 + j * 8 + 2 * t4 + 1];
+      gram[j][0] *= lo * c0;
+      gram[j][1] *= lo * c1;
+      gram[j][2] *= hi * c0;
+      gram[j][3] *= hi * c1;
+    }
+  }
+  float acc[8][4];                   // dQ (of the scaled q^) or dK: rows row_lo, row_hi, columns part * 64 + 8 j + 2 t4 (+ 1)
+#pragma unroll
+  for (int j = 0; j < 8; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
 
   for (int r = 0; r < rep; ++r) {
     const int hv = hq * rep + r;
     const size_t chunk = (static_cast<size_t>(batch) * gm.Hv + hv) * gm.N + n;
+    load_raw_tile<kBwdThreads>(mixed_b, gm, n, 2 * gm.Hqk * kD + hv * kD, sm.v);
+    load_chunk_tile(p.d_veff + chunk * kC * kD, sm.dxv);
+    load_chunk_tile(p.d_kq + chunk * 2 * kC * kD, sm.dxk);
     const float a_neg = -expf(p.A_log[hv]);
-    chunk_gates(p.b_in, p.a_in, a_neg, p.dt_bias[hv], gm, batch, n, hv, s_beta, s_g, s_G, s_eg, s_ed, s_asig);
-    if (tid < kC) s_dG[tid] = s_dbeta[tid] = 0.f;
-    {
-      float s[4][4], w[4][4];
-      gram_blocks(sq, sk, ti, tj, s, w);
+    float beta = 0.f, G = 0.f;
+    if (tid < kC) {
+      const int t = n * kC + tid;
+      float asig = 0.f;
+      if (t < gm.T) {
+        const size_t off = (tok0 + t) * gm.Hv + hv;
+        const float x = bf2f(p.a_in + off) + p.dt_bias[hv];
+        beta = sigmoid_f(bf2f(p.b_in + off));
+        G = a_neg * softplus_f(x);
+        asig = sigmoid_f(x);
+      }
+      sm.g[tid] = G;
+      sm.asig[tid] = asig;
+      sm.dG[tid] = 0.;
+      sm.dbeta[tid] = 0.f;
 #pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-          const int i = ti + 16 * a, j = tj + 16 * b;
-          const float D = j <= i ? expf(s_G[i] - s_G[j]) : 0.f;
-          sM0[i * kC + j] = j < i ? s[a][b] * D : 0.f;
-          sM1[i * kC + j] = j <= i ? w[a][b] * D : 0.f;
-        }
+      for (int o = 1; o < 32; o <<= 1) {
+        const float up = __shfl_up_sync(0xffffffffu, G, o);
+        if (lane >= o) G += up;
+      }
+      if (tid == 31) sm.warp0_sum = G;
     }
     __syncthreads();
-
-    float da[4][4];                            // dA of this thread's Gram entries
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int b = 0; b < 4; ++b) da[a][b] = 0.f;
-
-#pragma unroll 1
-    for (int h = 0; h < 2; ++h) {              // h = 0: the value columns, h = 1: the key columns of the solve
-      // The two substitutions of a pass are independent (X needs the right-hand side, Y the incoming gradient):
-      // threads 0-127 solve the columns of X while threads 128-255 solve the columns of Y.
-      if (tid < 128) {
-        const int c = tid;
-        float x[kC];
-        if (h == 0) {
-          const __nv_bfloat16* vp = mixed_b + 2 * gm.Hqk * kD + hv * kD + c;
-#pragma unroll
-          for (int i = 0; i < kC; ++i) {
-            const int t = n * kC + i;
-            x[i] = t < gm.T ? s_beta[i] * bf2f(vp + static_cast<size_t>(t) * gm.conv_dim) : 0.f;
-          }
-        } else {
-#pragma unroll
-          for (int i = 0; i < kC; ++i) x[i] = s_beta[i] * s_eg[i] * sk[i * kLd + c];
-        }
-        // X = (I + A)^-1 R with A_ij = beta_i M0_ij
-#pragma unroll
-        for (int i = 1; i < kC; ++i) {
-          float acc = 0.f;
-#pragma unroll
-          for (int j4 = 0; j4 * 4 < i; ++j4) {
-            const float4 m = *reinterpret_cast<const float4*>(sM0 + i * kC + 4 * j4);
-            acc += m.x * x[4 * j4] + m.y * x[4 * j4 + 1] + m.z * x[4 * j4 + 2] + m.w * x[4 * j4 + 3];
-          }
-          x[i] -= s_beta[i] * acc;
-        }
-#pragma unroll
-        for (int i = 0; i < kC; ++i) sX[i * kLd + c] = x[i];
-      } else {
-        const int c = tid - 128;
-        float x[kC];
-        // Y = (I + A)^-T dX, right-looking: once y_j is final, y_i -= A_ji y_j for every i < j
-        const __nv_bfloat16* dxp = h == 0 ? p.d_veff + chunk * kC * kD + c : p.d_kq + chunk * 2 * kC * kD + c;
-#pragma unroll
-        for (int i = 0; i < kC; ++i) x[i] = bf2f(dxp + i * kD);
-#pragma unroll
-        for (int j = kC - 1; j >= 1; --j) {
-          const float t = s_beta[j] * x[j];
-#pragma unroll
-          for (int i4 = 0; i4 * 4 < j; ++i4) {
-            const float4 m = *reinterpret_cast<const float4*>(sM0 + j * kC + 4 * i4);
-            x[4 * i4] -= m.x * t;
-            x[4 * i4 + 1] -= m.y * t;
-            x[4 * i4 + 2] -= m.z * t;
-            x[4 * i4 + 3] -= m.w * t;
-          }
-        }
-#pragma unroll
-        for (int i = 0; i < kC; ++i) sY[i * kLd + c] = x[i];
-        if (h == 0) {
-          __nv_bfloat16* dvp = d_mixed_b + 2 * gm.Hqk * kD + hv * kD + c;
-#pragma unroll
-          for (int i = 0; i < kC; ++i) {
-            const int t = n * kC + i;
-            if (t < gm.T) dvp[static_cast<size_t>(t) * gm.conv_dim] = __float2bfloat16(s_beta[i] * x[i]);
-          }
-        }
-      }
-      __syncthreads();
-      // dA -= Y X^T on this thread's entries
-#pragma unroll 2
-      for (int c = 0; c < kD; c += 4) {
-        float4 yi[4], xj[4];
-#pragma unroll
-        for (int a = 0; a < 4; ++a) {
-          yi[a] = *reinterpret_cast<const float4*>(sY + (ti + 16 * a) * kLd + c);
-          xj[a] = *reinterpret_cast<const float4*>(sX + (tj + 16 * a) * kLd + c);
-        }
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-          for (int b = 0; b < 4; ++b)
-            if (b <= a) da[a][b] -= dot4(yi[a], xj[b]);
-      }
-      // per-row dot products of Y with the right-hand side's own factor (v, or k^)
-      {
-        float u = 0.f;
-        const int t = n * kC + ri;
-        if (h == 0) {
-          if (t < gm.T) {
-            const __nv_bfloat16* vp = mixed_b + static_cast<size_t>(t) * gm.conv_dim + 2 * gm.Hqk * kD + hv * kD;
-#pragma unroll
-            for (int m = 0; m < 16; ++m) {
-              const float2 y2 = *reinterpret_cast<const float2*>(sY + ri * kLd + 2 * (rqd + 4 * m));
-              const float2 v2 = bf2f2(vp + 2 * (rqd + 4 * m));
-              u += y2.x * v2.x + y2.y * v2.y;
-            }
-          }
-        } else {
-#pragma unroll
-          for (int m = 0; m < 16; ++m) {
-            const float2 y2 = *reinterpret_cast<const float2*>(sY + ri * kLd + 2 * (rqd + 4 * m));
-            const float2 k2 = *reinterpret_cast<const float2*>(sk + ri * kLd + 2 * (rqd + 4 * m));
-            u += y2.x * k2.x + y2.y * k2.y;
-          }
-        }
-        u += __shfl_xor_sync(0xffffffffu, u, 1);
-        u += __shfl_xor_sync(0xffffffffu, u, 2);
-        if (rqd == 0) {
-          if (h == 0) {
-            atomicAdd(s_dbeta + ri, u);
-          } else {
-            atomicAdd(s_dbeta + ri, s_eg[ri] * u);
-            atomicAdd(s_dG + ri, s_beta[ri] * s_eg[ri] * u);
-          }
-        }
-      }
-      __syncthreads();
+    if (tid < kC) {
+      if (tid >= 32) G += sm.warp0_sum;
+      const float eg = expf(G);
+      sm.beta[tid] = beta;
+      sm.G[tid] = G;
+      sm.eg[tid] = eg;
+      sm.kscale[tid] = beta * eg * sm.rk[tid];
     }
-
-    // through the decayed Gram matrices: E = dA * A + d_intra * intra feeds dG (row sums minus column sums);
-    // dS = dA beta D and dW = d_intra D go to q^ and k^ through three 64 x 64 x 128 products
+    __syncthreads();
+    if (tid < kC) sm.ed[tid] = expf(sm.G[kC - 1] - sm.G[tid]);
     {
-      float m0[4][4], m1[4][4], di[4][4];
+      const float G_lo = sm.G[row_lo], G_hi = sm.G[row_hi], b_lo = sm.beta[row_lo], b_hi = sm.beta[row_hi];
+      double e_lo = 0., e_hi = 0.;
 #pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-          const int i = ti + 16 * a, j = tj + 16 * b;
-          m0[a][b] = sM0[i * kC + j];
-          m1[a][b] = sM1[i * kC + j];
-          di[a][b] = j <= i ? bf2f(p.d_intra + (chunk * kC + i) * kC + j) : 0.f;
+      for (int j = 0; j < 4; ++j) {
+        const int c0 = part * 32 + j * 8 + 2 * t4, c1 = c0 + 1;
+        const float2 Gc = *reinterpret_cast<const float2*>(sm.G + c0);
+        // decays, zero above the diagonal
+        const float d00 = c0 <= row_lo ? expf(G_lo - Gc.x) : 0.f, d01 = c1 <= row_lo ? expf(G_lo - Gc.y) : 0.f;
+        const float d10 = c0 <= row_hi ? expf(G_hi - Gc.x) : 0.f, d11 = c1 <= row_hi ? expf(G_hi - Gc.y) : 0.f;
+        if (second) {
+          // W = q^ k^T D: dW = d_intra D, and d_intra W feeds dG (row sums minus column sums)
+          const __nv_bfloat16* di = p.d_intra + chunk * kC * kC + c0;
+          const float2 i0 = bf2f2(di + row_lo * kC), i1 = bf2f2(di + row_hi * kC);
+          const float w00 = i0.x * d00, w01 = i0.y * d01, w10 = i1.x * d10, w11 = i1.y * d11;
+          *reinterpret_cast<float2*>(sm.W + row_lo * kTLd + c0) = make_float2(w00, w01);
+          *reinterpret_cast<float2*>(sm.W + row_hi * kTLd + c0) = make_float2(w10, w11);
+          const double x00 = w00 * gram[j][0], x01 = w01 * gram[j][1], x10 = w10 * gram[j][2], x11 = w11 * gram[j][3];
+          e_lo += x00 + x01;
+          e_hi += x10 + x11;
+          const double s0 = column_sum(x00 + x10), s1 = column_sum(x01 + x11);
+          if (g == 0) {
+            atomicAdd(sm.dG + c0, -s0);
+            atomicAdd(sm.dG + c1, -s1);
+          }
+        } else {
+          const float m00 = c0 < row_lo ? gram[j][0] * d00 : 0.f, m01 = c1 < row_lo ? gram[j][1] * d01 : 0.f;
+          const float m10 = c0 < row_hi ? gram[j][2] * d10 : 0.f, m11 = c1 < row_hi ? gram[j][3] * d11 : 0.f;
+          *reinterpret_cast<float2*>(sm.M0 + row_lo * kALd + c0) = make_float2(m00, m01);
+          *reinterpret_cast<float2*>(sm.M0 + row_hi * kALd + c0) = make_float2(m10, m11);
+          *reinterpret_cast<float2*>(sm.A + row_lo * kALd + c0) = make_float2(b_lo * m00, b_lo * m01);
+          *reinterpret_cast<float2*>(sm.A + row_hi * kALd + c0) = make_float2(b_hi * m10, b_hi * m11);
         }
-      __syncthreads();      // every entry is in registers before the mirrored writes start
-      float row_e[4], row_b[4];
+      }
+      if (second) {
+        e_lo = quad_sum(e_lo);
+        e_hi = quad_sum(e_hi);
+        if (t4 == 0) {
+          atomicAdd(sm.dG + row_lo, e_lo);
+          atomicAdd(sm.dG + row_hi, e_hi);
+        }
+      }
+    }
+    __syncthreads();
+    unit_lower_inverse<kBwdThreads>(sm.A, sm.T, sm.U);
+    {
+      // N = dX_v V^T diag(beta) + dX_k K^T diag(beta exp(G) / |k|): 16 columns per warp
+      const int c16 = (warp >> 2) * 16;
+      float nv[2][4], nk[2][4];
 #pragma unroll
-      for (int a = 0; a < 4; ++a) {
-        row_e[a] = row_b[a] = 0.f;
+      for (int j = 0; j < 2; ++j)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) {
-          const int i = ti + 16 * a, j = tj + 16 * b;
-          if (j > i) continue;               // the mirror entry's owner writes this position
-          const float D = expf(s_G[i] - s_G[j]);
-          const float dA = j < i ? da[a][b] : 0.f;
-          const float E = dA * s_beta[i] * m0[a][b] + di[a][b] * m1[a][b];
-          row_e[a] += E;
-          atomicAdd(s_dG + j, -E);
-          row_b[a] += dA * m0[a][b];
-          const float dS = dA * s_beta[i] * D;
-          const float dW = di[a][b] * D;
-          sM0[i * kC + j] = dS;
-          sM0[j * kC + i] = dS;
-          sM1[i * kC + j] = dW;
-          sM2[j * kC + i] = dW;
-          if (j < i) {
-            sM1[j * kC + i] = 0.f;
-            sM2[i * kC + j] = 0.f;
+        for (int e = 0; e < 4; ++e) nv[j][e] = nk[j][e] = 0.f;
+#pragma unroll
+      for (int ks = 0; ks < kD / 16; ++ks) {
+        const int ao = (mt * 16 + (lane & 15)) * kRawLd + ks * 16 + (lane >> 4) * 8;
+        const int bo = (c16 + (lane >> 4) * 8 + (lane & 7)) * kRawLd + ks * 16 + ((lane >> 3) & 1) * 8;
+        uint32_t a[4], b[4];
+        ldsm4(a, sm.dxv + ao);
+        ldsm4(b, sm.v + bo);
+        mma_add(nv[0], a, b[0], b[1]);
+        mma_add(nv[1], a, b[2], b[3]);
+        ldsm4(a, sm.dxk + ao);
+        ldsm4(b, sm.k + bo);
+        mma_add(nk[0], a, b[0], b[1]);
+        mma_add(nk[1], a, b[2], b[3]);
+      }
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const int c0 = c16 + j * 8 + 2 * t4;
+        const float2 sv = *reinterpret_cast<const float2*>(sm.beta + c0), sk = *reinterpret_cast<const float2*>(sm.kscale + c0);
+        *reinterpret_cast<float2*>(sm.N + row_lo * kALd + c0) =
+            make_float2(nv[j][0] * sv.x + nk[j][0] * sk.x, nv[j][1] * sv.y + nk[j][1] * sk.y);
+        *reinterpret_cast<float2*>(sm.N + row_hi * kALd + c0) =
+            make_float2(nv[j][2] * sv.x + nk[j][2] * sk.x, nv[j][3] * sv.y + nk[j][3] * sk.y);
+      }
+    }
+    {
+      // Y = T^T dX, 64 columns per warp in two halves. Values: dV = beta Y; keys: dK += beta exp(G) Y. The rows' products with the
+      // right-hand sides' own factors (v, k^) go to the gates.
+      auto t_transposed = [&](int row, int l) {
+        const float* t = sm.T + l * kTLd + mt * 16 + row;
+        return make_float2(t[0], t[kTLd]);
+      };
+      const float b_lo = sm.beta[row_lo], b_hi = sm.beta[row_hi], eb_lo = b_lo * sm.eg[row_lo], eb_hi = b_hi * sm.eg[row_hi];
+      float u_lo = 0.f, u_hi = 0.f;
+      const __nv_bfloat16* raw = second ? sm.k : sm.v;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int col = part * 64 + h * 32;
+        float y[4][4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) y[j][0] = y[j][1] = y[j][2] = y[j][3] = 0.f;
+        split_product<4>(y, t_transposed, mt, 4, (second ? sm.dxk : sm.dxv) + col);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int c = col + j * 8 + 2 * t4;
+          const float2 x0 = bf2f2(raw + row_lo * kRawLd + c), x1 = bf2f2(raw + row_hi * kRawLd + c);
+          u_lo += y[j][0] * x0.x + y[j][1] * x0.y;
+          u_hi += y[j][2] * x1.x + y[j][3] * x1.y;
+          if (second) {
+            acc[4 * h + j][0] += eb_lo * y[j][0];
+            acc[4 * h + j][1] += eb_lo * y[j][1];
+            acc[4 * h + j][2] += eb_hi * y[j][2];
+            acc[4 * h + j][3] += eb_hi * y[j][3];
+          } else {
+            __nv_bfloat16* dv = d_mixed_b + 2 * gm.Hqk * kD + hv * kD + c;
+            const int t = n * kC + row_lo;
+            if (t < gm.T) *reinterpret_cast<uint32_t*>(dv + static_cast<size_t>(t) * gm.conv_dim) = pack_bf16x2(b_lo * y[j][0], b_lo * y[j][1]);
+            if (t + 8 < gm.T) *reinterpret_cast<uint32_t*>(dv + static_cast<size_t>(t + 8) * gm.conv_dim) = pack_bf16x2(b_hi * y[j][2], b_hi * y[j][3]);
           }
         }
       }
+      u_lo = quad_sum(u_lo);
+      u_hi = quad_sum(u_hi);
+      if (t4 == 0) {
+        if (second) {
+          const float k_lo = u_lo * sm.rk[row_lo], k_hi = u_hi * sm.rk[row_hi];
+          atomicAdd(sm.dbeta + row_lo, sm.eg[row_lo] * k_lo);
+          atomicAdd(sm.dbeta + row_hi, sm.eg[row_hi] * k_hi);
+          atomicAdd(sm.dG + row_lo, static_cast<double>(eb_lo * k_lo));
+          atomicAdd(sm.dG + row_hi, static_cast<double>(eb_hi * k_hi));
+        } else {
+          atomicAdd(sm.dbeta + row_lo, u_lo);
+          atomicAdd(sm.dbeta + row_hi, u_hi);
+        }
+      }
+    }
+    __syncthreads();
+    // dA = -strict_lower(T^T N T^T): thread (ti, tj) owns rows ti, ti + 32 and columns tj + 16 b
+    const int ti = tid >> 4, tj = tid & 15;
+    {
+      float pr[2][4];
 #pragma unroll
-      for (int a = 0; a < 4; ++a) {
+      for (int a = 0; a < 2; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) pr[a][b] = 0.f;
+#pragma unroll
+      for (int lb = 0; lb < 4; ++lb)
+#pragma unroll
+        for (int l = lb * 16; l < lb * 16 + 16; l += 4) {   // T_jl = 0 for l > j
+          const float4 n0 = *reinterpret_cast<const float4*>(sm.N + ti * kALd + l), n1 = *reinterpret_cast<const float4*>(sm.N + (ti + 32) * kALd + l);
+#pragma unroll
+          for (int b = lb; b < 4; ++b) {
+            const float4 t = *reinterpret_cast<const float4*>(sm.T + (tj + 16 * b) * kTLd + l);
+            pr[0][b] += n0.x * t.x + n0.y * t.y + n0.z * t.z + n0.w * t.w;
+            pr[1][b] += n1.x * t.x + n1.y * t.y + n1.z * t.z + n1.w * t.w;
+          }
+        }
+#pragma unroll
+      for (int b = 0; b < 4; ++b) {
+        sm.P[ti * kTLd + tj + 16 * b] = pr[0][b];
+        sm.P[(ti + 32) * kTLd + tj + 16 * b] = pr[1][b];
+      }
+    }
+    __syncthreads();
+    {
+      float da[2][4];
+#pragma unroll
+      for (int a = 0; a < 2; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) da[a][b] = 0.f;
+#pragma unroll 4
+      for (int l = warp * 2; l < 32; ++l) {                 // T_li = 0 for i > l; rows ti < 32 have no columns from 32 on
+        const float t0 = sm.T[l * kTLd + ti];
+#pragma unroll
+        for (int b = 0; b < 2; ++b) da[0][b] = fmaf(-t0, sm.P[l * kTLd + tj + 16 * b], da[0][b]);
+      }
+#pragma unroll 4
+      for (int l = 32; l < kC; ++l) {
+        const float t0 = sm.T[l * kTLd + ti], t1 = sm.T[l * kTLd + ti + 32];
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+          const float x = sm.P[l * kTLd + tj + 16 * b];
+          if (b < 2) da[0][b] = fmaf(-t0, x, da[0][b]);
+          da[1][b] = fmaf(-t1, x, da[1][b]);
+        }
+      }
+      // dA A feeds dG (row sums minus column sums), dA M0 dbeta, dS = dA beta D the Gram matrix of k^
+#pragma unroll
+      for (int a = 0; a < 2; ++a) {
+        const int i = ti + 32 * a;
+        const float b_i = sm.beta[i], G_i = sm.G[i];
+        double row_e = 0.;
+        float row_b = 0.f;
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+          const int j = tj + 16 * b;
+          const bool low = j < i;
+          const float dA = low ? da[a][b] : 0.f, m0 = low ? sm.M0[i * kALd + j] : 0.f;
+          const float x = dA * m0;
+          const double E = x * b_i;
+          row_e += E;
+          row_b += x;
+          const double col = E + __shfl_xor_sync(0xffffffffu, E, 16);   // the two rows of the warp
+          if (lane < 16) atomicAdd(sm.dG + j, -col);
+          const float dS = low ? dA * b_i * expf(G_i - sm.G[j]) : 0.f;
+          if (j <= i) sm.S[i * kTLd + j] = dS;
+          if (low) sm.S[j * kTLd + i] = dS;
+        }
 #pragma unroll
         for (int o = 8; o >= 1; o >>= 1) {
-          row_e[a] += __shfl_xor_sync(0xffffffffu, row_e[a], o);
-          row_b[a] += __shfl_xor_sync(0xffffffffu, row_b[a], o);
+          row_e += __shfl_xor_sync(0xffffffffu, row_e, o);
+          row_b += __shfl_xor_sync(0xffffffffu, row_b, o);
         }
         if (tj == 0) {
-          atomicAdd(s_dG + ti + 16 * a, row_e[a]);
-          atomicAdd(s_dbeta + ti + 16 * a, row_b[a]);
+          atomicAdd(sm.dG + i, row_e);
+          atomicAdd(sm.dbeta + i, row_b);
         }
       }
     }
     __syncthreads();
-    float dq[32], dk[32];
     {
-      uint32_t v[32];
-      tmem_ld_32x32(park, v);
-      tmem_ld_wait();
-#pragma unroll
-      for (int m = 0; m < 32; ++m) dq[m] = __uint_as_float(v[m]);
-      tmem_ld_32x32(park + 32, v);
-      tmem_ld_wait();
-#pragma unroll
-      for (int m = 0; m < 32; ++m) {
-        const int i = 2 * m + hb;
-        dk[m] = __uint_as_float(v[m]) + s_beta[i] * s_eg[i] * sY[i * kLd + cc];   // sY: the key half of Y
+      // dQ += dW K^ + exp(G) dq_e;  dK += (dS + dS^T) K^ + dW^T Q^ + exp(G_end - G) dk_dec; the raw rows' norms scale the left side
+      const int col = part * 64;
+      if (second) {
+        auto s_left = [&](int row, int j) {
+          const float2 s = *reinterpret_cast<const float2*>(sm.S + (mt * 16 + row) * kTLd + j), rk = *reinterpret_cast<const float2*>(sm.rk + j);
+          return make_float2(s.x * rk.x, s.y * rk.y);
+        };
+        auto w_transposed = [&](int row, int j) {
+          const float* w = sm.W + j * kTLd + mt * 16 + row;
+          const float2 rq = *reinterpret_cast<const float2*>(sm.rq + j);
+          return make_float2(w[0] * rq.x, w[kTLd] * rq.y);
+        };
+        split_product<8>(acc, s_left, 0, 4, sm.k + col);
+        split_product<8>(acc, w_transposed, mt, 4, sm.q + col);
+      } else {
+        auto w_left = [&](int row, int j) {
+          const float2 w = *reinterpret_cast<const float2*>(sm.W + (mt * 16 + row) * kTLd + j), rk = *reinterpret_cast<const float2*>(sm.rk + j);
+          return make_float2(w.x * rk.x, w.y * rk.y);
+        };
+        split_product<8>(acc, w_left, 0, mt + 1, sm.k + col);
       }
-    }
-    {
-      float col[kC];
+      const __nv_bfloat16* grad = second ? p.d_kdec + chunk * kC * kD : p.d_kq + (chunk * 2 * kC + kC) * kD;
+      const __nv_bfloat16* raw = second ? sm.k : sm.q;
+      const float* dec = second ? sm.ed : sm.eg;
+      const float d_lo = dec[row_lo], d_hi = dec[row_hi];
+      float s_lo = 0.f, s_hi = 0.f;
 #pragma unroll
-      for (int j = 0; j < kC; ++j) col[j] = sk[j * kLd + cc];
-#pragma unroll
-      for (int m = 0; m < 32; ++m) {
-        const int i = 2 * m + hb;
-        float a0 = 0.f, a1 = 0.f;
-#pragma unroll
-        for (int j4 = 0; j4 < 16; ++j4) {
-          const float4 s4 = *reinterpret_cast<const float4*>(sM0 + i * kC + 4 * j4);
-          const float4 w4 = *reinterpret_cast<const float4*>(sM1 + i * kC + 4 * j4);
-          a0 += s4.x * col[4 * j4] + s4.y * col[4 * j4 + 1] + s4.z * col[4 * j4 + 2] + s4.w * col[4 * j4 + 3];
-          a1 += w4.x * col[4 * j4] + w4.y * col[4 * j4 + 1] + w4.z * col[4 * j4 + 2] + w4.w * col[4 * j4 + 3];
-        }
-        dk[m] += a0;
-        dq[m] += a1;
+      for (int j = 0; j < 8; ++j) {
+        const int c = col + j * 8 + 2 * t4;
+        const float2 g0 = bf2f2(grad + row_lo * kD + c), g1 = bf2f2(grad + row_hi * kD + c);
+        const float2 x0 = bf2f2(raw + row_lo * kRawLd + c), x1 = bf2f2(raw + row_hi * kRawLd + c);
+        s_lo += g0.x * x0.x + g0.y * x0.y;
+        s_hi += g1.x * x1.x + g1.y * x1.y;
+        acc[j][0] += d_lo * g0.x;
+        acc[j][1] += d_lo * g0.y;
+        acc[j][2] += d_hi * g1.x;
+        acc[j][3] += d_hi * g1.y;
       }
-#pragma unroll
-      for (int j = 0; j < kC; ++j) col[j] = sq[j * kLd + cc];
-#pragma unroll
-      for (int m = 0; m < 32; ++m) {
-        const int i = 2 * m + hb;
-        float a0 = 0.f;
-#pragma unroll
-        for (int j4 = 0; j4 < 16; ++j4) {
-          const float4 t4 = *reinterpret_cast<const float4*>(sM2 + i * kC + 4 * j4);
-          a0 += t4.x * col[4 * j4] + t4.y * col[4 * j4 + 1] + t4.z * col[4 * j4 + 2] + t4.w * col[4 * j4 + 3];
-        }
-        dk[m] += a0;
+      const float* norm = second ? sm.rk : sm.rq;
+      s_lo = quad_sum(s_lo) * norm[row_lo] * d_lo;
+      s_hi = quad_sum(s_hi) * norm[row_hi] * d_hi;
+      if (t4 == 0) {
+        atomicAdd(sm.dG + row_lo, static_cast<double>(second ? -s_lo : s_lo));
+        atomicAdd(sm.dG + row_hi, static_cast<double>(second ? -s_hi : s_hi));
+        if (second) atomicAdd(sm.dG + kC - 1, static_cast<double>(s_lo) + s_hi);
       }
-    }
-    // q_e = q^ exp(G), k_dec = k^ exp(G_end - G), e = exp(G_end)
-    {
-      const __nv_bfloat16* dqe = p.d_kq + (chunk * 2 * kC + kC) * kD;
-      const __nv_bfloat16* dkd = p.d_kdec + chunk * kC * kD;
-      float s1 = 0.f, s2 = 0.f;
-#pragma unroll
-      for (int m = 0; m < 16; ++m) {
-        const int c2 = 2 * (rqd + 4 * m);
-        const float2 g1 = bf2f2(dqe + ri * kD + c2), g2 = bf2f2(dkd + ri * kD + c2);
-        const float2 q2 = *reinterpret_cast<const float2*>(sq + ri * kLd + c2);
-        const float2 k2 = *reinterpret_cast<const float2*>(sk + ri * kLd + c2);
-        s1 += g1.x * q2.x + g1.y * q2.y;
-        s2 += g2.x * k2.x + g2.y * k2.y;
-      }
-      s1 += __shfl_xor_sync(0xffffffffu, s1, 1);
-      s1 += __shfl_xor_sync(0xffffffffu, s1, 2);
-      s2 += __shfl_xor_sync(0xffffffffu, s2, 1);
-      s2 += __shfl_xor_sync(0xffffffffu, s2, 2);
-      if (rqd == 0) {
-        const float t = s_ed[ri] * s2;
-        atomicAdd(s_dG + ri, s_eg[ri] * s1 - t);
-        atomicAdd(s_dG + kC - 1, t);
-      }
-      if (tid == 0) atomicAdd(s_dG + kC - 1, p.d_e[chunk] * s_eg[kC - 1]);
-#pragma unroll
-      for (int m = 0; m < 32; ++m) {
-        const int i = 2 * m + hb;
-        dq[m] += s_eg[i] * bf2f(dqe + i * kD + cc);
-        dk[m] += s_ed[i] * bf2f(dkd + i * kD + cc);
-      }
-    }
-    if (r + 1 < rep) {
-      uint32_t v[32];
-#pragma unroll
-      for (int m = 0; m < 32; ++m) v[m] = __float_as_uint(dq[m]);
-      tmem_st_32x32(park, v);
-#pragma unroll
-      for (int m = 0; m < 32; ++m) v[m] = __float_as_uint(dk[m]);
-      tmem_st_32x32(park + 32, v);
-      tmem_st_wait();
-    } else {
-      // last value head: straight to shared memory for the L2-norm backward (sX is free; sY still feeds nothing)
-#pragma unroll
-      for (int m = 0; m < 32; ++m) sX[(2 * m + hb) * kLd + cc] = dq[m];
-      __syncthreads();      // every thread has read the key half of Y out of sY
-#pragma unroll
-      for (int m = 0; m < 32; ++m) sY[(2 * m + hb) * kLd + cc] = dk[m];
+      if (tid == 0) atomicAdd(sm.dG + kC - 1, static_cast<double>(p.d_e[chunk] * sm.eg[kC - 1]));
     }
     __syncthreads();
     // gates: dg = reverse cumulative sum of dG; g = -exp(A_log) softplus(a + dt_bias); beta = sigmoid(b)
     if (tid < kC) {
-      float dg = 0.f;
-      for (int m = tid; m < kC; ++m) dg += s_dG[m];
+      double dg_sum = 0.;
+      for (int m = tid; m < kC; ++m) dg_sum += sm.dG[m];
+      const float dg = static_cast<float>(dg_sum);
       const int t = n * kC + tid;
       float d_alog = 0.f, d_dtb = 0.f;
       if (t < gm.T) {
         const size_t off = (tok0 + t) * gm.Hv + hv;
-        const float d_a = dg * a_neg * s_asig[tid];
-        const float beta = s_beta[tid];
+        const float d_a = dg * a_neg * sm.asig[tid], be = sm.beta[tid];
         p.d_a[off] = d_a;
-        p.d_b[off] = s_dbeta[tid] * beta * (1.f - beta);
-        d_alog = dg * s_g[tid];
+        p.d_b[off] = sm.dbeta[tid] * be * (1.f - be);
+        d_alog = dg * sm.g[tid];
         d_dtb = d_a;
       }
 #pragma unroll
@@ -861,46 +858,42 @@ __global__ void __launch_bounds__(kThreads, 1) gdn_chunk_prep_bwd_kernel(const P
     __syncthreads();
   }
 
-  // through the L2 norms: y = x r, r = rsqrt(sum x^2 + eps)  =>  dx = r (dy - y (y . dy))
+  // through the L2 norms: y = s x r, r = rsqrt(sum x^2 + eps), s = dk^-1/2 for q and 1 for k  =>  dx = s r dy - x r^2 (y . dy)
   {
-    float dotq = 0.f, dotk = 0.f;
+    const __nv_bfloat16* raw = second ? sm.k : sm.q;
+    const float* norm = second ? sm.rk : sm.rq;
+    float* dots = second ? sm.dotk : sm.dotq;
+    float s_lo = 0.f, s_hi = 0.f;
 #pragma unroll
-    for (int m = 0; m < 16; ++m) {
-      const int c2 = 2 * (rqd + 4 * m);
-      const float2 gq = *reinterpret_cast<const float2*>(sX + ri * kLd + c2);
-      const float2 gk = *reinterpret_cast<const float2*>(sY + ri * kLd + c2);
-      const float2 q2 = *reinterpret_cast<const float2*>(sq + ri * kLd + c2);
-      const float2 k2 = *reinterpret_cast<const float2*>(sk + ri * kLd + c2);
-      dotq += gq.x * q2.x + gq.y * q2.y;
-      dotk += gk.x * k2.x + gk.y * k2.y;
+    for (int j = 0; j < 8; ++j) {
+      const int c = part * 64 + j * 8 + 2 * t4;
+      const float2 x0 = bf2f2(raw + row_lo * kRawLd + c), x1 = bf2f2(raw + row_hi * kRawLd + c);
+      s_lo += acc[j][0] * x0.x + acc[j][1] * x0.y;
+      s_hi += acc[j][2] * x1.x + acc[j][3] * x1.y;
     }
-    dotq += __shfl_xor_sync(0xffffffffu, dotq, 1);
-    dotq += __shfl_xor_sync(0xffffffffu, dotq, 2);
-    dotk += __shfl_xor_sync(0xffffffffu, dotk, 1);
-    dotk += __shfl_xor_sync(0xffffffffu, dotk, 2);
-    const int t = n * kC + ri;
-    if (t < gm.T) {
-      const float rq = s_rq[ri], rk = s_rk[ri];
-      __nv_bfloat16* oq = d_mixed_b + static_cast<size_t>(t) * gm.conv_dim + hq * kD;
-      __nv_bfloat16* ok = oq + gm.Hqk * kD;
-      // sq holds q^ s (s = dk^-1/2): d q^ = s dQ, q^ (q^ . d q^) = sq (sq . dQ) / s
+    s_lo = quad_sum(s_lo);
+    s_hi = quad_sum(s_hi);
+    if (t4 == 0) {
+      atomicAdd(dots + row_lo, s_lo);
+      atomicAdd(dots + row_hi, s_hi);
+    }
+    __syncthreads();
+    // r = norm / s: r^2 (y . dy) = norm^3 / s^2 (x . dy)
+    const float inv_s2 = second ? 1.f : 1.f / (kQScale * kQScale);
+    const float n_lo = norm[row_lo], n_hi = norm[row_hi];
+    const float f_lo = n_lo * n_lo * n_lo * inv_s2 * dots[row_lo], f_hi = n_hi * n_hi * n_hi * inv_s2 * dots[row_hi];
+    const int t = n * kC + row_lo;
+    __nv_bfloat16* out = d_mixed_b + static_cast<size_t>(t) * gm.conv_dim + (second ? gm.Hqk * kD : 0) + hq * kD;
 #pragma unroll
-      for (int m = 0; m < 16; ++m) {
-        const int c2 = 2 * (rqd + 4 * m);
-        const float2 gq = *reinterpret_cast<const float2*>(sX + ri * kLd + c2);
-        const float2 gk = *reinterpret_cast<const float2*>(sY + ri * kLd + c2);
-        const float2 q2 = *reinterpret_cast<const float2*>(sq + ri * kLd + c2);
-        const float2 k2 = *reinterpret_cast<const float2*>(sk + ri * kLd + c2);
-        *reinterpret_cast<__nv_bfloat162*>(oq + c2) = __floats2bfloat162_rn(
-            rq * (kQScale * gq.x - q2.x * dotq / kQScale), rq * (kQScale * gq.y - q2.y * dotq / kQScale));
-        *reinterpret_cast<__nv_bfloat162*>(ok + c2) =
-            __floats2bfloat162_rn(rk * (gk.x - k2.x * dotk), rk * (gk.y - k2.y * dotk));
-      }
+    for (int j = 0; j < 8; ++j) {
+      const int c = part * 64 + j * 8 + 2 * t4;
+      const float2 x0 = bf2f2(raw + row_lo * kRawLd + c), x1 = bf2f2(raw + row_hi * kRawLd + c);
+      if (t < gm.T) *reinterpret_cast<uint32_t*>(out + c) = pack_bf16x2(n_lo * acc[j][0] - x0.x * f_lo, n_lo * acc[j][1] - x0.y * f_lo);
+      if (t + 8 < gm.T)
+        *reinterpret_cast<uint32_t*>(out + 8 * static_cast<size_t>(gm.conv_dim) + c) =
+            pack_bf16x2(n_hi * acc[j][2] - x1.x * f_hi, n_hi * acc[j][3] - x1.y * f_hi);
     }
   }
-  tc_fence_before();
-  __syncthreads();
-  if (tid < 32) tmem_dealloc(*s_tmem, 128);
 }
 
 bool prep_geom_ok(int B, int T, int Hqk, int Hv) { return B >= 1 && T >= 1 && Hqk >= 1 && Hv >= Hqk && Hv % Hqk == 0; }
@@ -933,7 +926,7 @@ cudaError_t launch_gdn_chunk_prep_bwd(const __nv_bfloat16* mixed, const __nv_bfl
                                       cudaStream_t stream) {
   if (!prep_geom_ok(B, T, Hqk, Hv)) return cudaErrorInvalidValue;
   const int N = (T + kC - 1) / kC;
-  constexpr int smem = kBwdSmemFloats * 4;
+  constexpr int smem = sizeof(PrepBwdSmem);
   static bool configured = false;
   if (!configured) {
     cudaError_t err = cudaFuncSetAttribute(gdn_chunk_prep_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -942,7 +935,7 @@ cudaError_t launch_gdn_chunk_prep_bwd(const __nv_bfloat16* mixed, const __nv_bfl
   }
   PrepBwdArgs args{mixed, b_in, a_in, A_log, dt_bias, d_kq, d_intra, d_kdec, d_veff, d_e,
                    d_mixed, d_b, d_a, d_A_log, d_dt_bias, {T, N, Hqk, Hv, (2 * Hqk + Hv) * kD}};
-  gdn_chunk_prep_bwd_kernel<<<dim3(N, Hqk, B), kThreads, smem, stream>>>(args);
+  gdn_chunk_prep_bwd_kernel<<<dim3(N, Hqk, B), kBwdThreads, smem, stream>>>(args);
   return cudaGetLastError();
 }
 

@@ -622,3 +622,37 @@ def test_fp8_quant_mx_kernel_matches_reference(cuda_device, transpose, block):
     assert torch.equal(sf.cpu(), sf_ref)
     assert torch.equal(q.cpu().view(torch.uint8), q_ref.view(torch.uint8))
 
+
+
+@pytest.mark.parametrize("B,T,n_qk,n_v", [(1, 1, 2, 4), (1, 65, 1, 1), (2, 171, 2, 16), (1, 640, 4, 8)])
+def test_chunk_prep_gradients_against_64_bits(cuda_device, B, T, n_qk, n_v):
+    """The gate parameters' gradients are 32-bit sums whose terms cancel a few hundredfold and whose exponentials are good to 2^-21: 1e-3.
+    The others are bf16: 2^-8."""
+    from jax_gpt_b200.models.qwen35 import deltanet as D
+    d, F = torch.float64, torch.nn.functional
+    g = torch.Generator(device=cuda_device).manual_seed(7)
+    rnd = lambda *s: torch.randn(*s, device=cuda_device, generator=g)
+    ins = (F.silu(rnd(B, T, (2 * n_qk + n_v) * 128)).bfloat16(), rnd(B, T, n_v).bfloat16(), rnd(B, T, n_v).bfloat16(),
+           torch.log(torch.rand(n_v, device=cuda_device, generator=g) * 4 + 0.1), torch.ones(n_v, device=cuda_device))
+    ins = [t.requires_grad_(True) for t in ins]
+    outs = D._GdnChunkPrepFn.apply(*ins, n_qk, n_v)
+    dys = [(torch.randn(o.shape, device=cuda_device, generator=g) * 0.1).to(o.dtype) for o in outs]
+    got = torch.autograd.grad(outs, ins, dys)
+
+    N, pad, kd = (T + 63) // 64, (-T) % 64, n_qk * 128
+    mixed, b, a, A_log, dt = ref_ins = [t.detach().to(d).requires_grad_(True) for t in ins]
+    unit = lambda x: x * torch.rsqrt(x.square().sum(-1, keepdim=True) + 1e-6)
+    heads = lambda x: unit(x.reshape(B, T, n_qk, 128)).repeat_interleave(n_v // n_qk, 2)
+    tiles = lambda x: F.pad(x.transpose(1, 2), (0, 0, 0, pad)).reshape(B * n_v, N, 64, 128)
+    gates = lambda x: F.pad(x.transpose(1, 2), (0, pad)).reshape(B * n_v, N, 64)
+    q, k, v = tiles(heads(mixed[..., :kd]) * 128 ** -0.5), tiles(heads(mixed[..., kd:2 * kd])), tiles(mixed[..., 2 * kd:].reshape(B, T, n_v, 128))
+    beta, G = gates(torch.sigmoid(b)), gates(-A_log.exp() * F.softplus(a + dt)).cumsum(-1)
+    decay, kb = torch.exp((G[..., :, None] - G[..., None, :]).tril()), k * beta[..., None]
+    A = ((kb @ k.transpose(-1, -2)) * decay).tril(-1)
+    x = torch.linalg.solve_triangular(torch.eye(64, device=cuda_device, dtype=d) + A,
+                                      torch.cat([v * beta[..., None], kb * torch.exp(G)[..., None]], -1), upper=False, unitriangular=True)
+    ref = [torch.cat([x[..., 128:], q * torch.exp(G)[..., None]], -2), ((q @ k.transpose(-1, -2)) * decay).tril(),
+           k * torch.exp(G[..., -1:] - G)[..., None], x[..., :128], torch.exp(G[..., -1])]
+    want = torch.autograd.grad([r.reshape(o.shape) for r, o in zip(ref, outs)], ref_ins, [y.to(d) for y in dys])
+    for x, y, bound in zip(got, want, (2.0 ** -8, 2.0 ** -8, 2.0 ** -8, 1e-3, 1e-3)):
+        assert _rel(x.to(d), y) < bound, (_rel(x, y), bound)
