@@ -859,12 +859,6 @@ __global__ void latent_merge_kernel(const float* __restrict__ part_o, const floa
 }
 
 // ---- experts -----------------------------------------------------------------------------------------------------
-__device__ __forceinline__ float clamped_glu(float g, float u, const GluArgs& a) {
-  g = fminf(g, a.limit);
-  u = fminf(fmaxf(u, -a.limit), a.limit);
-  return g * sigmoid_f(a.alpha * g) * (u + a.shift);
-}
-
 // The next expert in order of falling logits (equal ones by index) after expert `pi` with logit `pv`; -1: none left.
 // Called by a whole warp with uniform arguments; every lane gets the result.
 __device__ __forceinline__ int next_best(const float* z, int E, float pv, int pi, float& value) {

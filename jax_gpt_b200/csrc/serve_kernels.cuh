@@ -117,6 +117,18 @@ cudaError_t launch_moe_gather_rows(const __nv_bfloat16* x, const int* idx, const
                                    int M, int D, cudaStream_t st);
 cudaError_t launch_clamped_glu(const __nv_bfloat16* gu, const float* w_row, GluArgs glu, __nv_bfloat16* h, int rows, int I,
                                cudaStream_t st);
+// Grouped GEMM (grouped_gemm_sm100.cu): rows of expert e end at ends[e]. out (rows, cols); with the GLU the weights hold 2 * cols rows,
+// gate first, and w_row (optional) scales a row's gate and up. Strides in elements, multiples of 8.
+struct GroupedArgs {
+  const int* ends;
+  const float* w_row;
+  __nv_bfloat16* out;
+  GluArgs glu;
+  int K, cols, expert0, experts;   // the launch sets the last two
+  int* status;
+};
+cudaError_t launch_grouped_gemm(const __nv_bfloat16* xs, const __nv_bfloat16* w, int64_t w_row_stride, int64_t w_expert_stride,
+                                const GroupedArgs& args, bool glu, int rows, int n_experts, cudaStream_t st);
 cudaError_t launch_moe_combine_rows(const __nv_bfloat16* ys, const int* row_of, int top, float w, float* x, int M, int D,
                                     cudaStream_t st);
 

@@ -69,4 +69,23 @@ cudaError_t encode_tma_3d(CUtensorMap* map, const void* base, int elem_bytes, ui
   return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
+cudaError_t encode_tma_5d(CUtensorMap* map, const void* base, int elem_bytes, const uint64_t (&dims)[5], const uint64_t (&stride_bytes)[4],
+                          const uint32_t (&box)[5]) {
+  auto fn = get_encode();
+  if (fn == nullptr) return cudaErrorNotSupported;
+  ensure_context();
+  uint64_t low = reinterpret_cast<uintptr_t>(base);
+  cuuint64_t d[5], s[4];
+  cuuint32_t b[5], estr[5] = {1, 1, 1, 1, 1};
+  for (int i = 0; i < 5; ++i) {
+    d[i] = dims[i];
+    b[i] = box[i];
+    if (i < 4) low |= s[i] = stride_bytes[i];
+  }
+  if ((low & 15) != 0) return cudaErrorMisalignedAddress;
+  CUresult r = fn(map, dtype_for(elem_bytes), 5, const_cast<void*>(base), d, s, b, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+
 }  // namespace b200

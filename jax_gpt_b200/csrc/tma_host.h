@@ -26,4 +26,8 @@ cudaError_t encode_tma_3d(CUtensorMap* map, const void* base, int elem_bytes, ui
                           uint64_t outer, uint64_t mid_stride_bytes, uint64_t outer_stride_bytes, uint32_t box_inner,
                           uint32_t box_mid, uint32_t box_outer);
 
+// 5-D variant: extents from the innermost, byte strides of dimensions 1 to 4, box extents.
+cudaError_t encode_tma_5d(CUtensorMap* map, const void* base, int elem_bytes, const uint64_t (&dims)[5], const uint64_t (&stride_bytes)[4],
+                          const uint32_t (&box)[5]);
+
 }  // namespace b200

@@ -1,8 +1,8 @@
 """Gated expert layers whose experts are already chosen or scored, shared by the table and the router layers.
 
 Few tokens (decode), fp32 and odd widths run on two kernels that stream the chosen experts' rows and add straight into the
-fp32 result; larger bf16 batches sort the rows by expert on the device and run the library grouped GEMM (weights stored
-(E, out, in)) between gather, activation and combine kernels of csrc/serve_kernels.cu.
+fp32 result; larger bf16 batches sort the rows by expert on the device and run the grouped GEMMs of csrc/grouped_gemm_sm100.cu (weights
+stored (E, out, in), the activation in the first one's epilogue) between the gather and combine kernels of csrc/serve_kernels.cu.
 """
 from __future__ import annotations
 
@@ -37,6 +37,12 @@ def use_grouped(h, w_down, top: int) -> bool:
             and h.shape[0] * top >= GROUPED_MIN_ROWS)
 
 
+def _tileable(w):
+    """Weights the tensor maps can address: rows of unit stride whose starts are multiples of 16 bytes."""
+    ok = w.stride(2) == 1 and w.data_ptr() % 16 == 0 and all(s > 0 and s % 8 == 0 for s in w.stride()[:2])
+    return w if ok else w.clone(memory_format=torch.contiguous_format)
+
+
 def grouped_experts(h, idx, top: int, w_gate_up, w_down, glu: Glu, out, out_scale: float = 1.0, w_pair=None) -> torch.Tensor:
     """idx (M * top,) int32 experts; ``w_pair`` (M * top,) fp32 scales the experts' inputs, ``out_scale`` the summed output.
     Adds to ``out`` (M, D) fp32."""
@@ -51,10 +57,10 @@ def grouped_experts(h, idx, top: int, w_gate_up, w_down, glu: Glu, out, out_scal
     row_of = torch.empty(M * top, device=dev, dtype=torch.int32)
     w_row = torch.empty(M * top, device=dev, dtype=torch.float32) if w_pair is not None else None
     ops.moe_gather_rows(h, idx, pos, ends, counts, top, xs, row_of, w_pair, w_row)
-    gu = torch._grouped_mm(xs, w_gate_up.transpose(1, 2), offs=ends)
     act = torch.empty(M * top, I, device=dev, dtype=h.dtype)
-    ops.clamped_glu(gu, glu.limit, glu.alpha, glu.shift, w_row, act)
-    ys = torch._grouped_mm(act, w_down.transpose(1, 2), offs=ends)
+    ops.grouped_gemm(xs, _tileable(w_gate_up), ends, (glu.limit, glu.alpha, glu.shift), w_row, act)
+    ys = torch.empty(M * top, D, device=dev, dtype=h.dtype)
+    ops.grouped_gemm(act, _tileable(w_down), ends, None, None, ys)
     ops.moe_combine_rows(ys, row_of, top, out_scale, out)
     return out
 
